@@ -210,6 +210,31 @@ def test_vpt_pass_matches_oracle(ops, orc, w, h, n, hil, seed):
         assert_lists_match(got, want, lambda ids, xs, ys: packed_dist_np(sites, ids, xs, ys, inv), w, h)
 
 
+def lattice_sites(w, h, n, seed):
+    """Sites at whole pixels with unit softness and no anisotropy: with max(w, h) a power of
+    two every distance is exact in FP32 in any order of operations, so lists compare bit for
+    bit, and equal distances (decided by the order of arrival) are everywhere."""
+    rng = np.random.default_rng(seed)
+    s = np.zeros((n, 10), np.float32)
+    s[:, 0], s[:, 1] = rng.integers(0, w, n), rng.integers(0, h, n)
+    s[:, 3], s[:, 7] = rng.integers(1, 9, n), 1.0
+    s[::10, 0] = -1.0
+    return s
+
+
+@pytest.mark.parametrize("w,h,n,jump,inject", [(64, 40, 900, 1, 4), (33, 64, 500, 7, 3), (128, 5, 40, 64, 0),
+                                               (1, 16, 7, 1, 5), (64, 64, 3, 2, 1)])
+def test_vpt_ties_keep_the_order_of_arrival(ops, orc, w, h, n, jump, inject):
+    sites = lattice_sites(w, h, n, w + h + n)
+    c0, c1 = cases.random_field(w, h, n, n, empty_frac=0.1, dup_frac=0.2)
+    packed = orc.pack_sites(sites)
+    for i in range(3):  # random lists, then sorted ones
+        o0, o1 = ops.vpt_pass(t32(c0), t32(c1), tf(sites), 1.0 / max(w, h) ** 2, w, h, jump, 0, 1.0, inject, 0)
+        c0, c1 = orc.vpt_pass(c0, c1, packed, n, jump << 16, 0, w, h, 1.0, 0, inject)
+        np.testing.assert_array_equal(u32(o0), c0, err_msg=f"pass {i}")
+        np.testing.assert_array_equal(u32(o1), c1, err_msg=f"pass {i}")
+
+
 def test_vpt_pass_op(ops, orc):
     w, h, n = 48, 40, 500
     img, sites = cases.scene(w, h, n, 13)
