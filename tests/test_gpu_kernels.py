@@ -235,6 +235,19 @@ def test_vpt_ties_keep_the_order_of_arrival(ops, orc, w, h, n, jump, inject):
         np.testing.assert_array_equal(u32(o1), c1, err_msg=f"pass {i}")
 
 
+@pytest.mark.parametrize("w,h,n,step", [(64, 40, 900, 1), (33, 64, 500, 4), (128, 5, 40, 64), (1, 16, 7, 8),
+                                        (64, 64, 3, 2)])
+def test_jfa_ties_keep_the_order_of_arrival(ops, orc, w, h, n, step):
+    sites = lattice_sites(w, h, n, w + h + n)
+    f, _ = cases.random_field(w, h, n, n, empty_frac=0.1)
+    f[::7, 3] = f[::7, 0]  # repeated ids
+    for i in range(3):
+        out = torch.empty((w * h, 4), dtype=torch.int32, device="cuda")
+        got = u32(ops.jfa_flood(t32(f), out, tf(sites), 1.0 / max(w, h) ** 2, 0, step, 1, w, h))
+        f = orc.jfa_flood(f, sites, step, w, h)
+        np.testing.assert_array_equal(got, f, err_msg=f"pass {i}")
+
+
 def test_vpt_pass_op(ops, orc):
     w, h, n = 48, 40, 500
     img, sites = cases.scene(w, h, n, 13)
