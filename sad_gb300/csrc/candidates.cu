@@ -425,7 +425,7 @@ __device__ __forceinline__ VptQueue thread_queue(uint32_t* words) {
 }
 
 template <class Src>
-__global__ void __launch_bounds__(kVptThreads, 4) vpt_kernel(VptParams prm, Src src) {
+__global__ void __launch_bounds__(kVptThreads, 5) vpt_kernel(VptParams prm, Src src) {
     __shared__ uint32_t s_queue[kVptQueue * kVptThreads];
     pdl_wait();
     const int2 at = patch_pixel(blockIdx.x, blockIdx.y);
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(kVptThreads, 4) vpt_kernel(VptParams prm, Src 
 // block's image from the kernel parameters into shared memory (measured 3% faster than
 // reading them from the constant bank, unlike the gradient kernel, whose shared-memory
 // pipe is busy with the tile table's atomics).
-__global__ void __launch_bounds__(kVptThreads, 4)
+__global__ void __launch_bounds__(kVptThreads, 5)
     vpt_batch_kernel(const __grid_constant__ BatchArgs<VptBatchItem> a) {
     __shared__ uint32_t s_queue[kVptQueue * kVptThreads];
     pdl_wait();
