@@ -3,11 +3,11 @@
 //
 // Launch shape of the per-pixel kernels: 32x8 threads, one pixel per thread, so a warp
 // reads one 512-byte row segment of each candidate field (two 16-byte loads per lane).
-#include "accum.cuh"
 #include "common.cuh"
-#include "sources.cuh"
 #include "host_common.h"
 #include "kernels.h"
+#include "sources.cuh"
+#include "warp_sums.cuh"
 
 namespace sad {
 
@@ -196,46 +196,41 @@ void launch_clear_candidates(uint32_t* c0, uint32_t* c1, int w, int h, cudaStrea
 // ---------------------------------------------------------------------------
 // autograd adjoint (backends/pytorch/torch_ext/cuda/sad_bindings.cu:41-207)
 // ---------------------------------------------------------------------------
-// Key-table size per 256-pixel tile: 256 slots while sites are sparse enough (at most one
-// per four pixels: a tile then sees well under 200 distinct candidates), 512 above that.
-// Four blocks per SM (64 registers a thread) keep 32 warps resident for the latency of the
-// shared-memory atomics.
-template <class Src, int kBwdSlots>
+// Each warp takes an 8x4 patch and sums its sites' gradients by itself (warp_sums.cuh).  Bound
+// by issue (79% at 1999x1503): 327 us there with 46,941 sites and 44 us at 512x512 with 16,384,
+// against 875 and 93 us with a key table and float adds in shared memory.  Four blocks per SM
+// (64 registers): three and five are 6% and 2% slower.
+template <class Src>
 __global__ void __launch_bounds__(256, 4) render_backward_kernel(
     const uint4* __restrict__ cand0, const uint4* __restrict__ cand1,
     const float* __restrict__ grad_rgb, float* __restrict__ grad_sites, Src src, float inv_s2,
     uint32_t n, int w, int h, int cw, int ch) {
-    using Table = TileTable<10, kBwdSlots, AccFloat>;
-    auto& table = shared_table<Table>();
-    int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    table.init(tid, 256);
-    __syncthreads();
-
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
-    int y = blockIdx.y * blockDim.y + threadIdx.y;
-    bool inb = x < w && y < h;
-    float ux = static_cast<float>(x), uy = static_cast<float>(y);
-    float inv_scale = sqrtf(inv_s2);
+    const int lane = threadIdx.x, warp = threadIdx.y;
+    const int2 at = sum_patch_pixel(lane);
+    const int x = blockIdx.x * 32 + (warp & 3) * 8 + at.x;
+    const int y = blockIdx.y * 8 + (warp >> 2) * 4 + at.y;
+    const float ux = static_cast<float>(x), uy = static_cast<float>(y);
+    const float inv_scale = sqrtf(inv_s2);
     uint32_t ids[kCand];
     float wts[kCand];
     float3 pred = make_float3(0.f, 0.f, 0.f);
     float3 dLdp = make_float3(0.f, 0.f, 0.f);
-    uint32_t valid = 0;  // softmax members: id < n and !(position.x < 0)
-    uint32_t blend = 0;  // colour contributors: position.x >= 0
 #pragma unroll
     for (int i = 0; i < kCand; ++i) {
         ids[i] = kEmpty;
         wts[i] = 0.0f;
     }
-    if (inb) {
-        int p = y * w + x;
-        int ci = cand_index_for_pixel(x, y, w, h, cw, ch);
-        uint4 a = __ldg(cand0 + ci), b = __ldg(cand1 + ci);
+    if (x < w && y < h) {
+        const int p = y * w + x;
+        const int ci = cand_index_for_pixel(x, y, w, h, cw, ch);
+        const uint4 a = __ldg(cand0 + ci), b = __ldg(cand1 + ci);
         ids[0] = a.x; ids[1] = a.y; ids[2] = a.z; ids[3] = a.w;
         ids[4] = b.x; ids[5] = b.y; ids[6] = b.z; ids[7] = b.w;
         float logits[kCand];
         float3 cols[kCand];
         float mx = -INFINITY;
+        uint32_t valid = 0;  // softmax members: id < n and !(position.x < 0)
+        uint32_t blend = 0;  // colour contributors: position.x >= 0
 #pragma unroll
         for (int i = 0; i < kCand; ++i) {
             logits[i] = -INFINITY;
@@ -272,54 +267,24 @@ __global__ void __launch_bounds__(256, 4) render_backward_kernel(
             dLdp = make_float3(__ldg(grad_rgb + 3 * p), __ldg(grad_rgb + 3 * p + 1),
                                __ldg(grad_rgb + 3 * p + 2));
         }
+        // a weight that underflowed adds only zeros, unless its logit is not finite
+#pragma unroll
+        for (int i = 0; i < kCand; ++i)
+            if (!(valid >> i & 1u) || (wts[i] == 0.0f && logits[i] > -INFINITY)) ids[i] = kEmpty;
     }
-    int slots[kCand];
-#pragma unroll
-    for (int i = 0; i < kCand; ++i)
-        slots[i] = register_key(table, (valid >> i & 1u) ? ids[i] : kEmpty);
-    const uint32_t r = lane_rotation();
-    rotate8(ids, r);
-    rotate8(wts, r);
-    rotate8(slots, r);
-    const uint32_t vr = rotate_mask8(valid, r);
-#pragma unroll
-    for (int j = 0; j < kCand; ++j) {
-        if (!(vr >> j & 1u)) continue;
-        SiteGeom g;
-        float3 col;
-        src.load(ids[j], g, col);
-        float v[10];
-        candidate_grads(g, col, ux, uy, inv_s2, inv_scale, wts[j], dLdp, pred, false, v);
-        if (slots[j] >= 0) {
-            table.add(slots[j], v);
-        } else {
-            float* gs = grad_sites + static_cast<size_t>(ids[j]) * 10;
-#pragma unroll
-            for (int k = 0; k < 10; ++k) atomicAdd(gs + k, v[k]);
-        }
-    }
-    __syncthreads();
-    const int used = table.size();
-    for (int d = tid; d < used; d += 256) {
-        float* gs = grad_sites + static_cast<size_t>(table.key_at(d)) * 10;
-#pragma unroll
-        for (int k = 0; k < 10; ++k) atomicAdd(gs + k, table.value(k, d));
-    }
+    float rem[kCand];
+    add_site_gradients<false>(
+        ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred,
+        [&](uint32_t id, SiteGeom& g, float3& c) { src.load(id, g, c); },
+        [&](uint32_t id, int k, float v) { atomicAdd(grad_sites + static_cast<size_t>(id) * 10 + k, v); });
 }
 
 void launch_render_backward_raw(const uint32_t* c0, const uint32_t* c1, const float* grad_rgb,
                                 float* grad_sites, const Site* sites, float inv_s2, uint32_t n,
                                 int w, int h, int cw, int ch, cudaStream_t st) {
-    auto c0v = reinterpret_cast<const uint4*>(c0);
-    auto c1v = reinterpret_cast<const uint4*>(c1);
-    if (static_cast<double>(n) * 4.0 <= static_cast<double>(w) * h)
-        render_backward_kernel<RawSites, 256><<<pixel_grid(w, h), dim3(32, 8),
-                                                sizeof(TileTable<10, 256, AccFloat>), st>>>(
-            c0v, c1v, grad_rgb, grad_sites, RawSites{sites}, inv_s2, n, w, h, cw, ch);
-    else
-        render_backward_kernel<RawSites, 512><<<pixel_grid(w, h), dim3(32, 8),
-                                                sizeof(TileTable<10, 512, AccFloat>), st>>>(
-            c0v, c1v, grad_rgb, grad_sites, RawSites{sites}, inv_s2, n, w, h, cw, ch);
+    render_backward_kernel<RawSites><<<pixel_grid(w, h), dim3(32, 8), 0, st>>>(
+        reinterpret_cast<const uint4*>(c0), reinterpret_cast<const uint4*>(c1), grad_rgb, grad_sites,
+        RawSites{sites}, inv_s2, n, w, h, cw, ch);
     note_launches(1);
 }
 

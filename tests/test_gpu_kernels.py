@@ -104,6 +104,21 @@ def test_render_backward_matches_oracle(ops, orc, w, h, n, seed, field, log_tau)
     assert_grads_close(got.T, want.T, absw.T, want64=want64.T)
 
 
+@pytest.mark.parametrize("w,h,n", [(1, 1, 9), (3, 2, 9), (33, 9, 40), (31, 41, 200), (5, 64, 64)])
+def test_render_backward_at_patch_edges(ops, orc, w, h, n):
+    """Images that leave patches, groups and warps partly empty."""
+    img, sites = cases.scene(w, h, n, n)
+    sites[::7, 0] = -1.0
+    c0, c1 = cases.knn_field(sites, w, h)
+    c1[::3, 3] = c0[::3, 0]  # a repeated id
+    gout = np.random.default_rng(w).normal(size=(h, w, 3)).astype(np.float32)
+    got = ops.render_sad_backward(t32(c0), t32(c1), tf(sites), tf(gout), 1.0 / max(w, h) ** 2, w, h)
+    want, absw = orc.render_backward(c0, c1, sites, gout, w, h)
+    want64 = orc.render_backward_d(c0, c1, sites.astype(np.float64), gout.astype(np.float64), w, h,
+                                   1.0 / max(w, h) ** 2)
+    assert_grads_close(got.cpu().numpy().astype(np.float64).T, want.T, absw.T, want64=want64.T)
+
+
 def test_autograd_function_and_fp64_finite_differences(cuda, orc):
     """SADRenderFunction's backward against central differences (h = 1e-6) of the FP64
     forward on all per-site parameters (64x64, 256 sites, candidates fixed)."""
