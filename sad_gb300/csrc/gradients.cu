@@ -1,7 +1,7 @@
 // gradients.cu -- fused training gradient: forward softmax, dL/dpred of the MSE (+ SSIM)
-// loss, per-site parameter gradients and the prune removal delta, accumulated per 16x16
-// tile in a shared-memory table (accum.cuh): float for API calls, 64-bit fixed point
-// (bitwise reproducible) for the trainer.
+// loss, per-site parameter gradients and the prune removal delta.  The trainer's kernel
+// accumulates per 16x16 tile in a shared-memory table, in 64-bit fixed point (accum.cuh,
+// bitwise reproducible); the API's sums in the warp and adds floats (warp_sums.cuh).
 //
 // Semantics follow backends/cuda/src/gradients.cu:103-486 (computeGradientsTiledKernel):
 //   * masked pixels (mask <= 0) contribute nothing (the reference returns before its
@@ -11,20 +11,20 @@
 //   * the removal delta of a site is taken once per pixel with the site's summed weight
 //     over duplicate slots (gradients.cu:295-350).
 //
-// Tile mapping: 256 threads = 8 warps, each warp an 8x4 pixel patch, so the lanes of a
-// warp share most candidates and register each site with one CAS per warp.
+// Mapping: 256 threads = 8 warps, each warp an 8x4 pixel patch, so the lanes of a warp share
+// most candidates.
 #include "accum.cuh"
 #include "common.cuh"
 #include "host_common.h"
 #include "kernels.h"
 #include "sources.cuh"
+#include "warp_sums.cuh"
 
 #include <atomic>
 #include <type_traits>
 
 namespace sad {
 
-constexpr int kGradSlots = 512;  // hash slots (and values) of the in-kernel registration table
 constexpr float kRemovalSentinel = 1.0e6f;  // removal delta of a pixel the site dominates
 
 __device__ __forceinline__ float luma(const float* __restrict__ p) {
@@ -68,54 +68,24 @@ __device__ float ssim_dloss(const float* __restrict__ ren, const float* __restri
     return (dA * B + A * dB) / den - num * (dC * D + C * dD) / (den * den);
 }
 
-// Global fallback: float SoA arrays (API, accumulated like the reference) or the trainer's
-// [N][12] fixed-point records (slot 10 = removal delta, 11 = sentinel count).
-template <bool kFix, int NV>
+// Global fallback of the trainer's [N][12] fixed-point records (slot 10 = removal delta, 11 =
+// sentinel count).
+template <int NV>
 __device__ __forceinline__ void global_add(const GradParams& p, uint32_t key, const float (&v)[NV]) {
-    if constexpr (kFix) {
-        long long* o = p.fix12 + static_cast<size_t>(key) * 12;
+    long long* o = p.fix12 + static_cast<size_t>(key) * 12;
 #pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            const long long x = to_fix(v[k]);
-            if (x != 0) fix_add_global(o + k, x);  // a zero word leaves the sum as it is
-        }
-    } else {
-#pragma unroll
-        for (int k = 0; k < 10; ++k) atomicAdd(p.soa[k] + key, v[k]);
-        if constexpr (NV > 10) {
-            if (v[10] != 0.0f) atomicAdd(p.removal + key, v[10]);
-        }
+    for (int k = 0; k < NV; ++k) {
+        const long long x = to_fix(v[k]);
+        if (x != 0) fix_add_global(o + k, x);  // a zero word leaves the sum as it is
     }
 }
 
-template <bool kFix, int NV, class Table>
-__device__ __forceinline__ void flush_slot(const GradParams& p, const Table& table, int s) {
-    const uint32_t key = table.key_at(s);
-    if constexpr (kFix) {
-        long long* o = p.fix12 + static_cast<size_t>(key) * 12;
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            long long v = table.fixed(k, s);
-            if (v != 0) fix_add_global(o + k, v);
-        }
-    } else {
-#pragma unroll
-        for (int k = 0; k < 10; ++k) atomicAdd(p.soa[k] + key, table.value(k, s));
-        if constexpr (NV > 10) {
-            float r = table.value(10, s);
-            if (r != 0.0f) atomicAdd(p.removal + key, r);
-        }
-    }
-}
-
-// Values per table slot: 10 gradients, + removal delta (float path), + removal delta and
-// count of "keep < 1e-4" pixels (fixed-point path; each such pixel adds the reference's
-// 1e6 sentinel, kept as an exact integer count so the fixed-point sum cannot overflow).
-template <bool kFix, bool kRemoval>
+// Values per table entry of the trainer's kernel: 10 gradients, + removal delta and count of
+// "keep < 1e-4" pixels (each such pixel adds the reference's 1e6 sentinel, kept as an exact
+// integer count so the fixed-point sum cannot overflow).
+template <bool kRemoval>
 struct GradLayout {
-    static constexpr int NV = kRemoval ? (kFix ? 12 : 11) : 10;
-    using Mode = typename std::conditional<kFix, AccSplit, AccFloat>::type;
-    using Table = TileTable<NV, kGradSlots, Mode>;
+    static constexpr int NV = kRemoval ? 12 : 10;
     // precomputed registration (trainer): the tile's values, keys and staged sites, and
     // each thread's candidate weights (and removal deltas) for the accumulation loop
     struct Pre {
@@ -139,13 +109,14 @@ struct GradLayout {
 // with kRemoval, the removal delta on the first slot of each distinct valid site.
 // site(i, g, col) supplies candidate i's data.  Semantics of
 // backends/cuda/src/gradients.cu:103-300.
+// finite (nullable) receives the slots whose logit is finite.
 template <bool kRemoval, bool kSSIM, class SiteFn>
 __device__ __forceinline__ void pixel_forward(const GradParams& prm, int x, int y, float ux,
                                               float uy, float inv_s2, float inv_scale,
                                               const uint32_t (&ids)[kCand], float3 tgt,
                                               SiteFn site, float (&wts)[kCand],
                                               float (&rem)[kCand], uint32_t& valid,
-                                              float3& pred, float3& dLdp) {
+                                              float3& pred, float3& dLdp, uint32_t* finite = nullptr) {
     const uint32_t n = prm.site_count;
     uint32_t blend = 0;
     float logits[kCand];
@@ -169,6 +140,11 @@ __device__ __forceinline__ void pixel_forward(const GradParams& prm, int x, int 
     if (isinf(mx) && mx < 0.0f) {
         valid = 0;
         return;
+    }
+    if (finite) {
+#pragma unroll
+        for (int i = 0; i < kCand; ++i)
+            if (fabsf(logits[i]) < INFINITY) *finite |= 1u << i;
     }
     float sum = 0.0f;
 #pragma unroll
@@ -225,8 +201,8 @@ __device__ __forceinline__ void pixel_forward(const GradParams& prm, int x, int 
     }
 }
 
-// The 10 (+ removal) values one candidate adds; the removal slots follow the table mode.
-template <bool kFix, int NV>
+// The 10 (+ removal) values one candidate adds to the fixed-point sums.
+template <int NV>
 __device__ __forceinline__ void candidate_values(const SiteGeom& g, float3 col, float ux, float uy,
                                                  float inv_s2, float inv_scale, float w, float3 dLdp,
                                                  float3 pred, float rem, float removal_fix_mul,
@@ -236,30 +212,24 @@ __device__ __forceinline__ void candidate_values(const SiteGeom& g, float3 col, 
 #pragma unroll
     for (int k = 0; k < 10; ++k) v[k] = o[k];
     if constexpr (NV > 10) {
-        if constexpr (kFix) {
-            bool sentinel = rem == kRemovalSentinel;
-            v[10] = sentinel ? 0.0f : rem * removal_fix_mul;
-            v[11] = sentinel ? kFixInvScale : 0.0f;  // adds exactly 1
-        } else {
-            v[10] = rem;
-        }
+        bool sentinel = rem == kRemovalSentinel;
+        v[10] = sentinel ? 0.0f : rem * removal_fix_mul;
+        v[11] = sentinel ? kFixInvScale : 0.0f;  // adds exactly 1
     }
 }
 
-// One 16x16 tile per 256-thread block, each warp an 8x4 pixel patch, so the lanes of a
-// warp share most candidates.  Keys are registered here: one CAS per (warp, site).
-template <class Src, bool kFix, bool kRemoval, bool kSSIM>
-__global__ void __launch_bounds__(256, 3) fused_gradients_kernel(GradParams prm, Src src) {
-    using L = GradLayout<kFix, kRemoval>;
-    constexpr int NV = L::NV;
-    auto& table = shared_table<typename L::Table>();
-    const int tid = threadIdx.x;
-    table.init(tid, 256);
-    __syncthreads();
-
-    const int lane = tid & 31, warp = tid >> 5;
-    const int x = blockIdx.x * 16 + (warp & 1) * 8 + (lane & 7);
-    const int y = blockIdx.y * 16 + (warp >> 1) * 4 + (lane >> 3);
+// The API form, adding into the caller's float arrays: 32x8 pixels per block, an 8x4 patch per
+// warp, which sums its sites' gradients by itself (warp_sums.cuh).  Bound by issue.  A torch
+// step (render, gradients, tau diffusion, Adam, candidate refresh) at 768x512 with 24,576
+// sites takes 181 us, 276 us with a key table and float adds in shared memory; at 1237x941
+// with SSIM and removal deltas 332 instead of 555 us.  Four blocks per SM (64 registers):
+// three take 197 and 338 us.
+template <class Src, bool kRemoval, bool kSSIM>
+__global__ void __launch_bounds__(256, 4) fused_gradients_kernel(GradParams prm, Src src) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int2 at = sum_patch_pixel(lane);
+    const int x = blockIdx.x * 32 + (warp & 3) * 8 + at.x;
+    const int y = blockIdx.y * 8 + (warp >> 2) * 4 + at.y;
     const int w = prm.width, h = prm.height;
     const float inv_s2 = prm.inv_scale_sq;
     const float inv_scale = sqrtf(inv_s2);
@@ -268,7 +238,6 @@ __global__ void __launch_bounds__(256, 3) fused_gradients_kernel(GradParams prm,
     uint32_t ids[kCand];
     float wts[kCand];
     float rem[kCand];
-    uint32_t valid = 0;
     float3 pred = make_float3(0.f, 0.f, 0.f), dLdp = make_float3(0.f, 0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < kCand; ++i) {
@@ -287,48 +256,25 @@ __global__ void __launch_bounds__(256, 3) fused_gradients_kernel(GradParams prm,
         ids[4] = b.x; ids[5] = b.y; ids[6] = b.z; ids[7] = b.w;
         const float* t = prm.target + 3 * pix;
         float3 tgt = make_float3(__ldg(t), __ldg(t + 1), __ldg(t + 2));
+        uint32_t valid = 0, finite = 0;
         pixel_forward<kRemoval, kSSIM>(prm, x, y, ux, uy, inv_s2, inv_scale, ids, tgt,
                                        [&](int i, SiteGeom& g, float3& c) { src.load(ids[i], g, c); },
-                                       wts, rem, valid, pred, dLdp);
-    }
-
-    // 1. registration: one CAS per (warp, site)
-    int slots[kCand];
+                                       wts, rem, valid, pred, dLdp, &finite);
+        // a weight that underflowed adds only zeros, unless its logit is not finite
 #pragma unroll
-    for (int i = 0; i < kCand; ++i)
-        slots[i] = register_key(table, (valid >> i & 1u) ? ids[i] : kEmpty);
-
-    // 2. accumulate in a lane-rotated candidate order; the loop is kept rolled (the arrays
-    // shift down one entry per step) so the kernel body stays small in the instruction cache
-    const uint32_t r = lane_rotation();
-    rotate8(ids, r);
-    rotate8(wts, r);
-    rotate8(slots, r);
-    if constexpr (kRemoval) rotate8(rem, r);
-    uint32_t vr = rotate_mask8(valid, r);
-#pragma unroll 1
-    for (int j = 0; j < kCand; ++j) {
-        if (vr & 1u) {
-            SiteGeom g;
-            float3 col;
-            src.load(ids[0], g, col);
-            float v[NV];
-            candidate_values<kFix, NV>(g, col, ux, uy, inv_s2, inv_scale, wts[0], dLdp, pred, rem[0],
-                                       prm.removal_fix_mul, v);
-            if (slots[0] >= 0)
-                table.add(slots[0], v);
-            else
-                global_add<kFix, NV>(prm, ids[0], v);
-        }
-        vr >>= 1;
-        shift8(ids);
-        shift8(wts);
-        shift8(slots);
-        if constexpr (kRemoval) shift8(rem);
+        for (int i = 0; i < kCand; ++i)
+            if (!(valid >> i & 1u) || (wts[i] == 0.0f && rem[i] == 0.0f && (finite >> i & 1u))) ids[i] = kEmpty;
     }
-    __syncthreads();
-    const int used = table.size();
-    for (int d = tid; d < used; d += 256) flush_slot<kFix, NV>(prm, table, d);
+    add_site_gradients<kRemoval>(
+        ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred,
+        [&](uint32_t id, SiteGeom& g, float3& c) {
+            src.load(id, g, c);
+            if (!(g.l1 >= 1e-8f)) g.l2 = 1.0f / 1e-8f;  // l2 = 1 / max(l1, 1e-8) (gradients.cu:383)
+        },
+        [&](uint32_t id, int k, float v) {
+            float* to = k < 10 ? prm.soa[k < 10 ? k : 0] : prm.removal;
+            atomicAdd(to + id, v);
+        });
 }
 
 // Trainer form with the candidate field's registration precomputed (register_tiles_kernel):
@@ -361,7 +307,7 @@ __global__ void __launch_bounds__(256, 4)
 
 template <class Src, bool kRemoval, bool kSSIM>
 __device__ __forceinline__ void grad_pre_tile(const GradParams& prm, const Src& src, int bx, int by, int tiles_x) {
-    using L = GradLayout<true, kRemoval>;
+    using L = GradLayout<kRemoval>;
     constexpr int NV = L::NV;
     auto& sm = shared_table<typename L::Pre>();
     const int tid = threadIdx.x;
@@ -475,9 +421,9 @@ __device__ __forceinline__ void grad_pre_tile(const GradParams& prm, const Src& 
         float3 col;
         site_at(id, slot, g, col);
         float v[NV];
-        candidate_values<true, NV>(g, col, ux, uy, inv_s2, inv_scale, wt, dLdp, pred, rv, prm.removal_fix_mul, v);
+        candidate_values<NV>(g, col, ux, uy, inv_s2, inv_scale, wt, dLdp, pred, rv, prm.removal_fix_mul, v);
         if (slot < 0)
-            global_add<true, NV>(prm, id, v);
+            global_add<NV>(prm, id, v);
         else if (lanes)
             sm.lanes.add(slot, lane, v, prm.fix12, sm.dkey);
         else
@@ -592,20 +538,6 @@ void launch_register_tiles_batch(const RegisterBatchItem* items, const uint32_t*
     });
 }
 
-template <class Src, bool kFix, bool kRemoval, bool kSSIM>
-static void launch_fused(const GradParams& p, Src src, cudaStream_t st) {
-    dim3 grid((p.width + 15) / 16, (p.height + 15) / 16);
-    if constexpr (kFix) {
-        if (p.slot_map) {
-            launch_pdl(fused_gradients_pre_kernel<Src, kRemoval, kSSIM>, grid, dim3(256),
-                       sizeof(typename GradLayout<true, kRemoval>::Pre), st, p, src);
-            return;
-        }
-    }
-    fused_gradients_kernel<Src, kFix, kRemoval, kSSIM>
-        <<<grid, 256, sizeof(typename GradLayout<kFix, kRemoval>::Table), st>>>(p, src);
-}
-
 cudaError_t prepare_gradient_kernels();
 
 // Opt-in of the >48 KB shared-memory launches, once per device (an attribute set, not a
@@ -619,63 +551,60 @@ static void ensure_gradient_kernels() {
     if (prepare_gradient_kernels() == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
 }
 
-template <class Src, bool kFix>
-static void dispatch_gradients(const GradParams& p, Src src, cudaStream_t st) {
-    ensure_gradient_kernels();
-    bool rem = p.compute_removal != 0;
-    bool ssim = p.ssim_weight > 0.0f;
-    if (rem && ssim)
-        launch_fused<Src, kFix, true, true>(p, src, st);
-    else if (rem)
-        launch_fused<Src, kFix, true, false>(p, src, st);
+// launch(removal, ssim) with both as compile-time constants.
+template <class Launch>
+static void dispatch_gradients(bool removal, bool ssim, Launch launch) {
+    if (removal && ssim)
+        launch(std::true_type{}, std::true_type{});
+    else if (removal)
+        launch(std::true_type{}, std::false_type{});
     else if (ssim)
-        launch_fused<Src, kFix, false, true>(p, src, st);
+        launch(std::false_type{}, std::true_type{});
     else
-        launch_fused<Src, kFix, false, false>(p, src, st);
+        launch(std::false_type{}, std::false_type{});
     note_launches(1);
 }
 
-template <class Src, bool kFix, bool kRemoval>
+template <bool kRemoval, bool kSSIM>
 static cudaError_t allow_variant() {
-    size_t smem = sizeof(typename GradLayout<kFix, kRemoval>::Table);
-    cudaError_t e = allow_dynamic_smem(fused_gradients_kernel<Src, kFix, kRemoval, false>, smem);
-    if (e == cudaSuccess) e = allow_dynamic_smem(fused_gradients_kernel<Src, kFix, kRemoval, true>, smem);
-    if constexpr (kFix) {
-        size_t pre = sizeof(typename GradLayout<true, kRemoval>::Pre);
-        if (e == cudaSuccess) e = allow_dynamic_smem(fused_gradients_pre_kernel<Src, kRemoval, false>, pre);
-        if (e == cudaSuccess) e = allow_dynamic_smem(fused_gradients_pre_kernel<Src, kRemoval, true>, pre);
-        if constexpr (std::is_same<Src, PreparedSites>::value) {
-            if (e == cudaSuccess) e = allow_dynamic_smem(fused_gradients_batch_kernel<Src, kRemoval, false>, pre);
-            if (e == cudaSuccess) e = allow_dynamic_smem(fused_gradients_batch_kernel<Src, kRemoval, true>, pre);
-        }
-    }
+    constexpr size_t pre = sizeof(typename GradLayout<kRemoval>::Pre);
+    cudaError_t e = allow_dynamic_smem(fused_gradients_pre_kernel<PreparedSites, kRemoval, kSSIM>, pre);
+    if (e == cudaSuccess) e = allow_dynamic_smem(fused_gradients_batch_kernel<PreparedSites, kRemoval, kSSIM>, pre);
     return e;
 }
 
 cudaError_t prepare_gradient_kernels() {
-    cudaError_t e = allow_variant<RawSites, false, true>();
-    if (e == cudaSuccess) e = allow_variant<PreparedSites, false, true>();
-    if (e == cudaSuccess) e = allow_variant<PreparedSites, true, false>();
-    if (e == cudaSuccess) e = allow_variant<PreparedSites, true, true>();
+    cudaError_t e = allow_variant<false, false>();
+    if (e == cudaSuccess) e = allow_variant<false, true>();
+    if (e == cudaSuccess) e = allow_variant<true, false>();
+    if (e == cudaSuccess) e = allow_variant<true, true>();
     return e;
 }
 
 void launch_gradients_raw(const GradParams& p, const Site* sites, cudaStream_t st) {
-    dispatch_gradients<RawSites, false>(p, RawSites{sites}, st);
+    const dim3 grid((p.width + 31) / 32, (p.height + 7) / 8);
+    dispatch_gradients(p.compute_removal != 0, p.ssim_weight > 0.0f, [&](auto removal, auto ssim) {
+        fused_gradients_kernel<RawSites, decltype(removal)::value, decltype(ssim)::value>
+            <<<grid, 256, 0, st>>>(p, RawSites{sites});
+    });
 }
 
+// The trainer's form: p.fix12 and a registered candidate field.
 void launch_gradients_prepared(const GradParams& p, const SiteGeom* geom, const SiteColor* color,
                                cudaStream_t st) {
-    if (p.fix12)
-        dispatch_gradients<PreparedSites, true>(p, PreparedSites{geom, color}, st);
-    else
-        dispatch_gradients<PreparedSites, false>(p, PreparedSites{geom, color}, st);
+    ensure_gradient_kernels();
+    const dim3 grid((p.width + 15) / 16, (p.height + 15) / 16);
+    dispatch_gradients(p.compute_removal != 0, p.ssim_weight > 0.0f, [&](auto removal, auto ssim) {
+        constexpr bool kRemoval = decltype(removal)::value, kSSIM = decltype(ssim)::value;
+        launch_pdl(fused_gradients_pre_kernel<PreparedSites, kRemoval, kSSIM>, grid, dim3(256),
+                   sizeof(typename GradLayout<kRemoval>::Pre), st, p, PreparedSites{geom, color});
+    });
 }
 
 template <bool kRemoval, bool kSSIM>
 static void launch_batch_variant(const BatchArgs<GradBatchItem>& a, uint32_t tiles, cudaStream_t st) {
     launch_pdl(fused_gradients_batch_kernel<PreparedSites, kRemoval, kSSIM>, dim3(tiles), dim3(256),
-               sizeof(typename GradLayout<true, kRemoval>::Pre), st, a);
+               sizeof(typename GradLayout<kRemoval>::Pre), st, a);
 }
 
 void launch_gradients_batch(const GradBatchItem* items, const uint32_t* tile_prefix, uint32_t n_items,

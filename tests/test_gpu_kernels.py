@@ -306,6 +306,29 @@ def test_fused_gradients_match_oracle(ops, orc, w, h, n, removal, masked, ssim):
         assert np.all(np.abs(r - rem) <= 1e-3 * np.maximum(np.abs(rem), 1.0) + 1e-4)
 
 
+@pytest.mark.parametrize("w,h,n,removal,ssim", [(1, 1, 9, True, 0.0), (3, 2, 9, False, 0.2), (33, 9, 40, True, 0.0),
+                                                (31, 41, 200, True, 0.2), (5, 64, 64, False, 0.0)])
+def test_fused_gradients_at_patch_edges(ops, orc, w, h, n, removal, ssim):
+    """Nearest-site fields on images that leave patches, groups and warps partly empty."""
+    img, sites = cases.scene(w, h, n, n)
+    sites[::7, 0] = -1
+    c0, c1 = cases.knn_field(sites, w, h)
+    c1[::3, 3] = c0[::3, 0]  # a repeated id
+    mask = np.ones((h, w), np.float32)
+    mask[:, w // 2: w // 2 + 1] = 0.0 if w > 1 else 1.0
+    rendered = orc.render(c0, c1, sites, w, h)
+    bufs = _grad_buffers(n)
+    ops.compute_gradients_tiled(t32(c0), t32(c1), tf(img), tf(rendered), tf(mask), tf(sites), *bufs,
+                                1.0 / max(w, h) ** 2, 0, int(removal), ssim, w, h)
+    g, a, rem = orc.compute_gradients(c0, c1, img, sites, w, h, mask=mask, rendered=rendered, ssim_weight=ssim,
+                                      removal=removal)
+    want64 = orc.compute_gradients_d(c0, c1, img, sites, w, h, mask) if ssim == 0 else None
+    assert_grads_close(np.stack([b.cpu().numpy() for b in bufs[:10]]).astype(np.float64), g, a, want64=want64)
+    if removal:
+        r = bufs[10].cpu().numpy().astype(np.float64)
+        assert np.all(np.abs(r - rem) <= 1e-3 * np.maximum(np.abs(rem), 1.0) + 1e-4)
+
+
 def _fixed_gradients(w, h, n, c0, c1, img, rendered, mask, sites, removal, ssim):
     """The trainer's fixed-point gradient kernel through sad_compute_gradients_fixed:
     (int64 [N,12] sums, removal scale)."""
