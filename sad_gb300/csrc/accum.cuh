@@ -212,17 +212,19 @@ struct TileValues<NV, N, AccSplit> {
 //     each entry has four copies;
 //   wide (up to kTileKeys entries): block = 2 * (entry / kNarrowKeys) + row parity, so each
 //     entry has two copies.
-// Both address a word as block * kStride + value * kNarrowKeys + entry % kNarrowKeys, so
-// one accumulation loop serves both.  Adds follow TileValues<.., AccSplit>::add_unique (at
+// Both address a word as block * kStride + value * kRow + entry % kNarrowKeys, so one
+// accumulation loop serves both; rows of kNarrowKeys + 1 words put the values of one entry in
+// different banks, where the flush reads them side by side.  Adds follow TileValues<.., AccSplit>::add_unique (at
 // most one add per pixel and entry: a copy sums at most 128 single-word terms of |x| <=
 // 2^22); the hi words (rare) are shared.
 constexpr int kNarrowKeys = kTileKeys / 2;
 
 template <int NV>
 struct TileWords {
-    static constexpr int kStride = NV * kNarrowKeys + 8;  // blocks 8 banks apart
+    static constexpr int kRow = kNarrowKeys + 1;
+    static constexpr int kStride = (NV * kRow + 31) / 32 * 32 + 8;  // blocks 8 banks apart
     int lo[4 * kStride];
-    int hi[NV][kTileKeys];
+    int hi[NV][kTileKeys + 1];
 
     // the row bits of a lane in pixel row `row` (0-3) of its warp patch, and the block of
     // entry d for those bits (a narrow tile's entries are all below kNarrowKeys)
@@ -238,7 +240,7 @@ struct TileWords {
 #pragma unroll
         for (int k = 0; k < NV; ++k) {
             hi[k][d] = 0;
-            for (int b = b0; b < b0 + nb; ++b) word(b, d)[k * kNarrowKeys] = 0;
+            for (int b = b0; b < b0 + nb; ++b) word(b, d)[k * kRow] = 0;
         }
     }
     __device__ __forceinline__ void add_unique(int d, int block, const float (&v)[NV]) {
@@ -249,13 +251,13 @@ struct TileWords {
         if (m < 0.25f) {
 #pragma unroll
             for (int k = 0; k < NV; ++k)
-                atomicAdd(lc + k * kNarrowKeys, __float_as_int(fmaf(v[k], kFixScale, 12582912.0f)) - 0x4B400000);
+                atomicAdd(lc + k * kRow, __float_as_int(fmaf(v[k], kFixScale, 12582912.0f)) - 0x4B400000);
         } else {
 #pragma unroll
             for (int k = 0; k < NV; ++k) {
                 int h, l;
                 split_fix(v[k], h, l);
-                atomicAdd(lc + k * kNarrowKeys, l);
+                atomicAdd(lc + k * kRow, l);
                 if (h != 0) atomicAdd(&hi[k][d], h);
             }
         }
@@ -263,7 +265,7 @@ struct TileWords {
     __device__ __forceinline__ long long fixed(int k, int d, bool wide) const {
         const int b0 = wide ? (d / kNarrowKeys) << 1 : 0, nb = wide ? 2 : 4;
         long long x = static_cast<long long>(hi[k][d]) * (1ll << kSplitLoBits);
-        for (int b = b0; b < b0 + nb; ++b) x += static_cast<long long>(word(b, d)[k * kNarrowKeys]);
+        for (int b = b0; b < b0 + nb; ++b) x += static_cast<long long>(word(b, d)[k * kRow]);
         return x;
     }
 };

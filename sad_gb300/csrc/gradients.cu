@@ -434,13 +434,12 @@ __device__ __forceinline__ void grad_pre_tile(const GradParams& prm, const Src& 
         sm.lanes.flush(used, tid, prm.fix12, sm.dkey);
         return;
     }
-    for (int d = tid; d < used; d += 256) {
-        long long* o = prm.fix12 + static_cast<size_t>(sm.dkey[d]) * 12;
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            const long long x = sm.vals.fixed(k, d, wide);
-            if (x != 0) fix_add_global(o + k, x);
-        }
+    // (entry, value) pairs in order: neighbouring lanes add to neighbouring words of a record,
+    // so an instruction touches a third of the sectors that one entry per lane would
+    for (int q = tid; q < used * NV; q += 256) {
+        const int d = q / NV, k = q - d * NV;
+        const long long x = sm.vals.fixed(k, d, wide);
+        if (x != 0) fix_add_global(prm.fix12 + static_cast<size_t>(sm.dkey[d]) * 12 + k, x);
     }
 }
 
