@@ -332,6 +332,48 @@ struct LaneWords {
     }
 };
 
+// The terms of a crowded tile (kTileCrowded), which has no table: about one term per site and
+// warp, added to the global records.  A warp lays the 64-bit words of its 32 candidates out in
+// shared memory and adds them word by word, neighbouring lanes to neighbouring words of a
+// record: a third of the sectors per instruction of one record per lane.  Bound by the 64-bit
+// adds in L2: in the third window of a 1024x1024 fit the gradient kernel takes 262 us (334 us
+// with a table and its overflow added lane by lane), the registration 64 us (239 us).
+template <int NV>
+struct TermWords {
+    long long w[8][32][NV + 1];  // rows of an odd number of words, for the banks
+
+    __device__ __forceinline__ void put(int warp, int lane, const float (&v)[NV]) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            int h, l;
+            split_fix(v[k], h, l);
+            w[warp][lane][k] = static_cast<long long>(h) * (1ll << kSplitLoBits) + l;
+        }
+    }
+    // all lanes of the warp; adds: the lane has put its words, for site id
+    __device__ __forceinline__ void flush(int warp, int lane, bool adds, uint32_t id, long long* fix12) {
+        const uint32_t members = __ballot_sync(0xffffffffu, adds);
+        if (members == 0u) return;
+        __syncwarp();
+        int rec = lane / NV, k = lane % NV;  // pair lane + 32 j of the 32 x NV
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const uint32_t key = __shfl_sync(0xffffffffu, id, rec);
+            if (members >> rec & 1u) {
+                const long long x = w[warp][rec][k];
+                if (x != 0) fix_add_global(fix12 + static_cast<size_t>(key) * 12 + k, x);
+            }
+            rec += 32 / NV;
+            k += 32 % NV;
+            if (k >= NV) {
+                k -= NV;
+                ++rec;
+            }
+        }
+        __syncwarp();
+    }
+};
+
 // Keys and values of one tile (keys registered in the kernel).
 template <int NV, int SLOTS, class Mode>
 struct TileTable : KeyTable<SLOTS>, TileValues<NV, SLOTS, Mode> {
@@ -395,18 +437,17 @@ __device__ __forceinline__ uint32_t lane_rotation() {
     return ((l & 7u) * 5u + (l >> 3) * 2u) & 7u;
 }
 
-// Registration of one pixel's candidate list into its tile's table (all 32 lanes of the
-// warp call it); writes the packed 8 x u16 table indices (0xFFFF: none) to the slot map and
-// returns how many of them name an entry at or past kNarrowKeys (a far entry: keys are
-// claimed nearest candidate first, so those are the tile's far, low-weight candidates).
-template <class Table, class Map>
-__device__ __forceinline__ int register_tile_pixel(Table& table, const uint32_t (&ids)[8],
-                                                   uint32_t n, int x, int y, int w, bool inside,
-                                                   const Map& map) {
-    uint32_t packed[4] = {0u, 0u, 0u, 0u};
+// Registration of candidates FROM .. TO - 1 of one pixel into its tile's table (all 32 lanes
+// of the warp call it): adds their packed u16 table indices (0xFFFF: none) to the pixel's
+// slot-map words and returns how many of them name an entry at or past kNarrowKeys (a far
+// entry: keys are claimed nearest candidate first, so those are the tile's far, low-weight
+// candidates).
+template <int FROM, int TO, class Table>
+__device__ __forceinline__ int register_tile_pixel(Table& table, const uint32_t (&ids)[8], uint32_t n,
+                                                   uint32_t (&packed)[4]) {
     int far = 0;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = FROM; i < TO; ++i) {
         int slot = register_key(table, ids[i] < n ? ids[i] : kEmpty);
         // a repeated id in the list takes the global path, so a pixel adds at most once
         // to each table entry (TileValues::add_unique)
@@ -417,9 +458,7 @@ __device__ __forceinline__ int register_tile_pixel(Table& table, const uint32_t 
         far += (sidx != 0xFFFFu && sidx >= static_cast<uint32_t>(kNarrowKeys)) ? 1 : 0;
         packed[i >> 1] |= sidx << (16 * (i & 1));
     }
-    if (inside)
-        map.slot_map[static_cast<size_t>(y) * w + x] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-    return inside ? far : 0;
+    return far;
 }
 
 // A tile's word-table shape (TileWords): wide when more than `rule` of its (pixel,
@@ -431,6 +470,11 @@ __device__ __forceinline__ int register_tile_pixel(Table& table, const uint32_t 
 constexpr int kWideFarRefs = 256;
 // tile_count word: keys in use, plus this flag for a wide tile
 constexpr int kTileWideFlag = 1 << 30;
+// A crowded tile: its first two candidates per pixel already name more than kTileKeys sites
+// (the random lists that a fit starts from, or several sites per pixel).  No table would hold
+// its keys, so the registration stops there and the gradient kernel adds its terms to global
+// memory directly.
+constexpr int kTileCrowded = 1 << 29;
 
 // After the tile's registrations (and a barrier): its key list, and its key count with the
 // shape flag (far_refs: the tile's summed register_tile_pixel results).

@@ -52,10 +52,11 @@ struct sad_batch {
     uint32_t* site_prefix = nullptr;
     cudaStream_t st = nullptr, side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_done = nullptr;
-    cudaGraphExec_t graphs[2][2][3] = {};
-    uint64_t graph_kernels[2][2][3] = {};  // kernel launches one replay runs
-    cudaGraphExec_t wgraphs[3] = {};  // a whole refresh window per start field (as the trainer's)
-    uint64_t wgraph_kernels[3] = {};
+    cudaGraphExec_t graphs[3][2][2][3] = {};  // as the trainer's
+    uint64_t graph_kernels[3][2][2][3] = {};  // kernel launches one replay runs
+    cudaGraphExec_t wgraphs[3][3] = {};       // a whole refresh window per stage and start field
+    uint64_t wgraph_kernels[3][3] = {};
+    int crowd_end = 0, stage = 0;  // crowd_stage(), the last image's end for all
     std::vector<cudaEvent_t> tev;
     size_t tev_used = 0;
 };
@@ -63,18 +64,16 @@ struct sad_batch {
 namespace {
 
 void drop_batch_graphs(sad_batch* b) {
-    for (auto& x : b->graphs)
-        for (auto& y : x)
-            for (auto& g : y)
-                if (g) {
-                    cudaGraphExecDestroy(g);
-                    g = nullptr;
-                }
-    for (auto& g : b->wgraphs)
-        if (g) {
-            cudaGraphExecDestroy(g);
-            g = nullptr;
-        }
+    auto drop = [](cudaGraphExec_t& g) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    };
+    for (auto& stage : b->graphs)
+        for (auto& upd : stage)
+            for (auto& prune : upd)
+                for (auto& g : prune) drop(g);
+    for (auto& stage : b->wgraphs)
+        for (auto& g : stage) drop(g);
 }
 
 uint32_t tiles_of(const sad_trainer* t) { return static_cast<uint32_t>(((t->w + 15) / 16) * ((t->h + 15) / 16)); }
@@ -221,14 +220,14 @@ void batch_iteration(sad_batch* b, bool upd, bool prune, int field, cudaStream_t
         cudaStreamWaitEvent(b->side, b->ev_fork, 0);
         launch_pack_geom_batch(b->site_items, b->site_prefix, B, b->site_grid, b->side);
         launch_vpt_batch(b->vpt_items[field].data(), b->vpt_prefix.data(), B, b->side);
-        launch_register_tiles_batch(b->reg_items[next].data(), b->tile_prefix.data(), B, b->side);
+        launch_register_tiles_batch(b->reg_items[next].data(), b->tile_prefix.data(), B, b->stage == 0, b->side);
         cudaEventRecord(b->ev_join, b->side);
     }
     const bool timed = b->timing && b->tev_used + 2 <= b->tev.size();
     if (timed) cudaEventRecord(b->tev[b->tev_used], s);
     {
         NvtxRange r("batch: gradients");
-        launch_gradients_batch(b->grad_items[field].data(), b->tile_prefix.data(), B, prune, false, s);
+        launch_gradients_batch(b->grad_items[field].data(), b->tile_prefix.data(), B, prune, false, b->stage < 2, s);
     }
     if (timed) {
         cudaEventRecord(b->tev[b->tev_used + 1], s);
@@ -380,6 +379,8 @@ extern "C" sad_status_t sad_batch_init(sad_batch_t* b) {
         SAD_TRY(check_cuda(cudaStreamSynchronize(t->st), "sad_batch_init: trainer sync"));
     }
     drop_batch_graphs(b);
+    b->crowd_end = 0;
+    for (sad_trainer* t : b->tr) b->crowd_end = std::max(b->crowd_end, t->crowd_end);
     SAD_TRY(build_tables(b));
     SAD_TRY(check_cuda(cudaStreamSynchronize(b->st), "sad_batch_init: sync"));
     b->iter = 0;
@@ -411,9 +412,10 @@ extern "C" sad_status_t sad_batch_run(sad_batch_t* b, int end) {
     NvtxRange r(eager ? "batch iterations (eager)" : "batch iterations (graph replays)");
     for (int it = b->iter; it < end; ++it) {
         const IterPlan& p = plan[it];
+        b->stage = crowd_stage(b->crowd_end, std::max(1, b->cfg.cand_update_freq), it);
         if (!eager && batch_window_at(b, plan, it, end)) {
-            cudaGraphExec_t& g = b->wgraphs[b->cur];
-            uint64_t& nk = b->wgraph_kernels[b->cur];
+            cudaGraphExec_t& g = b->wgraphs[b->stage][b->cur];
+            uint64_t& nk = b->wgraph_kernels[b->stage][b->cur];
             if (!g) SAD_TRY(capture_batch_window(b, b->cur, &g, &nk));
             SAD_TRY(check_cuda(cudaGraphLaunch(g, b->st), "batch graph launch"));
             note_launches(nk);
@@ -426,8 +428,8 @@ extern "C" sad_status_t sad_batch_run(sad_batch_t* b, int end) {
         if (eager) {
             batch_iteration(b, p.upd, p.prune, b->cur, b->st);
         } else {
-            cudaGraphExec_t& g = b->graphs[p.upd][p.prune][b->cur];
-            uint64_t& nk = b->graph_kernels[p.upd][p.prune][b->cur];
+            cudaGraphExec_t& g = b->graphs[b->stage][p.upd][p.prune][b->cur];
+            uint64_t& nk = b->graph_kernels[b->stage][p.upd][p.prune][b->cur];
             if (!g) SAD_TRY(capture_batch(b, p.upd, p.prune, b->cur, &g, &nk));
             SAD_TRY(check_cuda(cudaGraphLaunch(g, b->st), "batch graph launch"));
             note_launches(nk);

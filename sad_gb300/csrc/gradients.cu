@@ -92,6 +92,7 @@ struct GradLayout {
         union {
             TileWords<NV> vals;   // lo words per pixel row (narrow tiles) or row parity (wide)
             LaneWords<NV> lanes;  // words per warp lane (tiles of at most kLaneKeys entries)
+            TermWords<NV> terms;  // words of one candidate per lane (crowded tiles)
         };
         uint32_t dkey[kTileKeys];
         // staged site records of the first kNarrowKeys entries (the entries of a wide tile
@@ -103,6 +104,7 @@ struct GradLayout {
         float rem[kRemoval ? kCand : 1][256];
     };
     static_assert(sizeof(LaneWords<NV>) <= sizeof(TileWords<NV>), "the lane words reuse the tile words' memory");
+    static_assert(sizeof(TermWords<NV>) <= sizeof(TileWords<NV>), "the term words reuse the tile words' memory");
 };
 
 // Forward of one pixel: softmax over the 8 candidates, pred, dL/dpred (+ SSIM term) and,
@@ -282,30 +284,31 @@ __global__ void __launch_bounds__(256, 4) fused_gradients_kernel(GradParams prm,
 // cleared and their sites staged in shared memory in one pass, and the accumulation loop
 // reads each candidate's table index, weight and site data by index instead of carrying
 // rotated register arrays.
-template <class Src, bool kRemoval, bool kSSIM>
+// kCrowded: the field's registration may have marked tiles as crowded.
+template <class Src, bool kRemoval, bool kSSIM, bool kCrowded>
 __device__ __forceinline__ void grad_pre_tile(const GradParams& prm, const Src& src, int bx, int by, int tiles_x);
 
-template <class Src, bool kRemoval, bool kSSIM>
+template <class Src, bool kRemoval, bool kSSIM, bool kCrowded>
 __global__ void __launch_bounds__(256, 4) fused_gradients_pre_kernel(GradParams prm, Src src) {
     pdl_wait();
-    grad_pre_tile<Src, kRemoval, kSSIM>(prm, src, blockIdx.x, blockIdx.y, gridDim.x);
+    grad_pre_tile<Src, kRemoval, kSSIM, kCrowded>(prm, src, blockIdx.x, blockIdx.y, gridDim.x);
 }
 
 // Batched form: one launch over the tiles of up to kBatchLaunchItems images, passed by
 // value.  Every thread finds its block's image in the constant bank, and grad_pre_tile
 // reads that image's parameters from there.
-template <class Src, bool kRemoval, bool kSSIM>
+template <class Src, bool kRemoval, bool kSSIM, bool kCrowded>
 __global__ void __launch_bounds__(256, 4)
     fused_gradients_batch_kernel(const __grid_constant__ BatchArgs<GradBatchItem> a) {
     pdl_wait();
     const uint32_t i = a.item_of(blockIdx.x);
     const GradBatchItem& it = a.items[i];
     const int local = static_cast<int>(blockIdx.x - a.block_prefix[i]);
-    grad_pre_tile<Src, kRemoval, kSSIM>(it.p, Src{it.geom, it.color}, local % it.tiles_x, local / it.tiles_x,
-                                        it.tiles_x);
+    grad_pre_tile<Src, kRemoval, kSSIM, kCrowded>(it.p, Src{it.geom, it.color}, local % it.tiles_x,
+                                                  local / it.tiles_x, it.tiles_x);
 }
 
-template <class Src, bool kRemoval, bool kSSIM>
+template <class Src, bool kRemoval, bool kSSIM, bool kCrowded>
 __device__ __forceinline__ void grad_pre_tile(const GradParams& prm, const Src& src, int bx, int by, int tiles_x) {
     using L = GradLayout<kRemoval>;
     constexpr int NV = L::NV;
@@ -313,9 +316,10 @@ __device__ __forceinline__ void grad_pre_tile(const GradParams& prm, const Src& 
     const int tid = threadIdx.x;
     const int tile = by * tiles_x + bx;
     const int tile_word = prm.tile_count[tile];
+    const bool crowded = kCrowded && tile_word == kTileCrowded;  // no table: used is 0, every slot -1
     const bool wide = (tile_word & kTileWideFlag) != 0;  // uniform over the block
     // a narrow tile keeps its first kNarrowKeys entries; slot_of() sends the rest global
-    const int used = wide ? tile_word & ~kTileWideFlag : min(tile_word, kNarrowKeys);
+    const int used = crowded ? 0 : wide ? tile_word & ~kTileWideFlag : min(tile_word, kNarrowKeys);
     // the lane-word shape (uniform over the block; every shape gives the same sums)
     const bool lanes = !wide && tile_word <= kLaneKeys;
     if (lanes) sm.lanes.zero(used, tid);
@@ -370,8 +374,10 @@ __device__ __forceinline__ void grad_pre_tile(const GradParams& prm, const Src& 
     int ci = 0;
     if (live && prm.mask) live = __ldg(prm.mask + pix) > 0.0f;
     if (live) {
-        uint4 m = __ldg(prm.slot_map + pix);
-        pm[0] = m.x; pm[1] = m.y; pm[2] = m.z; pm[3] = m.w;
+        if (!crowded) {
+            uint4 m = __ldg(prm.slot_map + pix);
+            pm[0] = m.x; pm[1] = m.y; pm[2] = m.z; pm[3] = m.w;
+        }
         ci = cand_index_for_pixel(x, y, w, h, prm.cand_width, prm.cand_height);
         uint32_t ids[kCand];
         uint4 a = __ldg(reinterpret_cast<const uint4*>(prm.cand0) + ci);
@@ -400,6 +406,30 @@ __device__ __forceinline__ void grad_pre_tile(const GradParams& prm, const Src& 
     // banks), or with lane words in the same order in every lane (broadcast record loads)
     const uint32_t r = lanes ? 0u : lane_rotation();
     const int rbits = TileWords<NV>::row_bits(lane >> 3, wide);
+    if (crowded) {
+#pragma unroll 1
+        for (int c = 0; c < kCand; ++c) {
+            bool adds = (valid >> c & 1u) != 0u;
+            uint32_t id = kEmpty;
+            if (adds) {
+                const float wt = sm.wts[c][tid];
+                const float rv = kRemoval ? sm.rem[kRemoval ? c : 0][tid] : 0.0f;
+                adds = !(wt == 0.0f && rv == 0.0f);  // as below
+                if (adds) {
+                    id = (c < 4 ? prm.cand0 : prm.cand1)[4 * static_cast<size_t>(ci) + (c & 3)];
+                    SiteGeom g;
+                    float3 col;
+                    src.load(id, g, col);
+                    float v[NV];
+                    candidate_values<NV>(g, col, ux, uy, inv_s2, inv_scale, wt, dLdp, pred, rv, prm.removal_fix_mul,
+                                         v);
+                    sm.terms.put(warp, lane, v);
+                }
+            }
+            sm.terms.flush(warp, lane, adds, id, prm.fix12);
+        }
+        return;
+    }
 #pragma unroll 1
     for (int j = 0; j < kCand; ++j) {
         const int c = static_cast<int>((j + r) & 7u);
@@ -449,19 +479,21 @@ __device__ __forceinline__ void grad_pre_tile(const GradParams& prm, const Src& 
 // n is registered; inactive sites simply receive no value.
 __device__ __forceinline__ void register_tile(const uint4* __restrict__ c0, const uint4* __restrict__ c1,
                                               uint32_t n, int w, int h, int cw, int ch, const TileMap& map,
-                                              int bx, int by, int tiles_x);
+                                              bool may_crowd, int bx, int by, int tiles_x);
 
 __global__ void __launch_bounds__(256) register_tiles_kernel(const uint4* __restrict__ c0,
                                                              const uint4* __restrict__ c1, uint32_t n,
-                                                             int w, int h, int cw, int ch, TileMap map) {
+                                                             int w, int h, int cw, int ch, TileMap map,
+                                                             bool may_crowd) {
     pdl_wait();
-    register_tile(c0, c1, n, w, h, cw, ch, map, blockIdx.x, blockIdx.y, gridDim.x);
+    register_tile(c0, c1, n, w, h, cw, ch, map, may_crowd, blockIdx.x, blockIdx.y, gridDim.x);
 }
 
 // Batched form over the tiles of up to kBatchLaunchItems images (by value, as the gradient
 // kernel's); one thread copies the block's image into shared memory, which measured faster
 // here than constant-bank reads.
-__global__ void __launch_bounds__(256) register_tiles_batch_kernel(const __grid_constant__ BatchArgs<RegisterBatchItem> a) {
+__global__ void __launch_bounds__(256) register_tiles_batch_kernel(const __grid_constant__ BatchArgs<RegisterBatchItem> a,
+                                                                  bool may_crowd) {
     pdl_wait();
     __shared__ RegisterBatchItem s_it;
     __shared__ int s_local;
@@ -473,12 +505,12 @@ __global__ void __launch_bounds__(256) register_tiles_batch_kernel(const __grid_
     __syncthreads();
     const int tx = s_it.tiles_x;
     register_tile(reinterpret_cast<const uint4*>(s_it.c0), reinterpret_cast<const uint4*>(s_it.c1), s_it.n, s_it.w,
-                  s_it.h, s_it.cw, s_it.ch, s_it.map, s_local % tx, s_local / tx, tx);
+                  s_it.h, s_it.cw, s_it.ch, s_it.map, may_crowd, s_local % tx, s_local / tx, tx);
 }
 
 __device__ __forceinline__ void register_tile(const uint4* __restrict__ c0, const uint4* __restrict__ c1,
                                               uint32_t n, int w, int h, int cw, int ch, const TileMap& map,
-                                              int bx, int by, int tiles_x) {
+                                              bool may_crowd, int bx, int by, int tiles_x) {
     __shared__ KeyTable<512> table;
     __shared__ int s_far;  // the tile's references to far entries
     const int tid = threadIdx.x;
@@ -499,7 +531,20 @@ __device__ __forceinline__ void register_tile(const uint4* __restrict__ c0, cons
 #pragma unroll
         for (int i = 0; i < kCand; ++i) ids[i] = kEmpty;
     }
-    const int far = __reduce_add_sync(0xffffffffu, register_tile_pixel(table, ids, n, x, y, w, inside, map));
+    uint32_t packed[4] = {0u, 0u, 0u, 0u};
+    int far = register_tile_pixel<0, 2>(table, ids, n, packed);
+    if (may_crowd) {
+        __syncthreads();
+        const bool crowded = table.size() > kTileKeys;
+        __syncthreads();  // the table grows again below
+        if (crowded) {
+            if (tid == 0) map.tile_count[by * tiles_x + bx] = kTileCrowded;
+            return;
+        }
+    }
+    far += register_tile_pixel<2, 8>(table, ids, n, packed);
+    if (inside) map.slot_map[static_cast<size_t>(y) * w + x] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+    far = __reduce_add_sync(0xffffffffu, inside ? far : 0);
     if (lane == 0 && far != 0) atomicAdd(&s_far, far);
     __syncthreads();
     const int rule = map.wide_far_refs ? *map.wide_far_refs : kWideFarRefs;
@@ -522,17 +567,17 @@ TileMap tile_map_at(uint32_t* base, int w, int h) {
 }
 
 void launch_register_tiles(const uint32_t* c0, const uint32_t* c1, uint32_t n, int w, int h,
-                           int cw, int ch, const TileMap& map, cudaStream_t st) {
+                           int cw, int ch, const TileMap& map, bool may_crowd, cudaStream_t st) {
     dim3 grid((w + 15) / 16, (h + 15) / 16);
     launch_pdl(register_tiles_kernel, grid, dim3(256), 0, st, reinterpret_cast<const uint4*>(c0),
-               reinterpret_cast<const uint4*>(c1), n, w, h, cw, ch, map);
+               reinterpret_cast<const uint4*>(c1), n, w, h, cw, ch, map, may_crowd);
     note_launches(1);
 }
 
 void launch_register_tiles_batch(const RegisterBatchItem* items, const uint32_t* tile_prefix, uint32_t n_items,
-                                 cudaStream_t st) {
+                                 bool may_crowd, cudaStream_t st) {
     for_each_batch_launch(items, tile_prefix, n_items, [&](const BatchArgs<RegisterBatchItem>& a, uint32_t tiles) {
-        launch_pdl(register_tiles_batch_kernel, dim3(tiles), dim3(256), 0, st, a);
+        launch_pdl(register_tiles_batch_kernel, dim3(tiles), dim3(256), 0, st, a, may_crowd);
         note_launches(1);
     });
 }
@@ -550,74 +595,73 @@ static void ensure_gradient_kernels() {
     if (prepare_gradient_kernels() == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
 }
 
-// launch(removal, ssim) with both as compile-time constants.
-template <class Launch>
-static void dispatch_gradients(bool removal, bool ssim, Launch launch) {
-    if (removal && ssim)
-        launch(std::true_type{}, std::true_type{});
-    else if (removal)
-        launch(std::true_type{}, std::false_type{});
-    else if (ssim)
-        launch(std::false_type{}, std::true_type{});
-    else
-        launch(std::false_type{}, std::false_type{});
-    note_launches(1);
+// f(flag) with the flag as a compile-time constant.
+template <class F>
+static auto with_constant(bool flag, F f) {
+    return flag ? f(std::true_type{}) : f(std::false_type{});
 }
 
-template <bool kRemoval, bool kSSIM>
-static cudaError_t allow_variant() {
-    constexpr size_t pre = sizeof(typename GradLayout<kRemoval>::Pre);
-    cudaError_t e = allow_dynamic_smem(fused_gradients_pre_kernel<PreparedSites, kRemoval, kSSIM>, pre);
-    if (e == cudaSuccess) e = allow_dynamic_smem(fused_gradients_batch_kernel<PreparedSites, kRemoval, kSSIM>, pre);
+// The trainer's two gradient kernels over each combination of their switches.
+template <class F>
+static cudaError_t each_gradient_variant(F f) {
+    cudaError_t e = cudaSuccess;
+    for (int bits = 0; bits < 8 && e == cudaSuccess; ++bits)
+        e = with_constant(bits & 1, [&](auto removal) {
+            return with_constant(bits & 2, [&](auto ssim) {
+                return with_constant(bits & 4, [&](auto crowded) { return f(removal, ssim, crowded); });
+            });
+        });
     return e;
 }
 
 cudaError_t prepare_gradient_kernels() {
-    cudaError_t e = allow_variant<false, false>();
-    if (e == cudaSuccess) e = allow_variant<false, true>();
-    if (e == cudaSuccess) e = allow_variant<true, false>();
-    if (e == cudaSuccess) e = allow_variant<true, true>();
-    return e;
+    return each_gradient_variant([](auto removal, auto ssim, auto crowded) {
+        constexpr size_t pre = sizeof(typename GradLayout<removal>::Pre);
+        cudaError_t e = allow_dynamic_smem(fused_gradients_pre_kernel<PreparedSites, removal, ssim, crowded>, pre);
+        if (e == cudaSuccess)
+            e = allow_dynamic_smem(fused_gradients_batch_kernel<PreparedSites, removal, ssim, crowded>, pre);
+        return e;
+    });
 }
 
 void launch_gradients_raw(const GradParams& p, const Site* sites, cudaStream_t st) {
     const dim3 grid((p.width + 31) / 32, (p.height + 7) / 8);
-    dispatch_gradients(p.compute_removal != 0, p.ssim_weight > 0.0f, [&](auto removal, auto ssim) {
-        fused_gradients_kernel<RawSites, decltype(removal)::value, decltype(ssim)::value>
-            <<<grid, 256, 0, st>>>(p, RawSites{sites});
+    with_constant(p.compute_removal != 0, [&](auto removal) {
+        with_constant(p.ssim_weight > 0.0f, [&](auto ssim) {
+            fused_gradients_kernel<RawSites, removal, ssim><<<grid, 256, 0, st>>>(p, RawSites{sites});
+        });
     });
+    note_launches(1);
 }
 
 // The trainer's form: p.fix12 and a registered candidate field.
-void launch_gradients_prepared(const GradParams& p, const SiteGeom* geom, const SiteColor* color,
+void launch_gradients_prepared(const GradParams& p, const SiteGeom* geom, const SiteColor* color, bool may_crowd,
                                cudaStream_t st) {
     ensure_gradient_kernels();
     const dim3 grid((p.width + 15) / 16, (p.height + 15) / 16);
-    dispatch_gradients(p.compute_removal != 0, p.ssim_weight > 0.0f, [&](auto removal, auto ssim) {
-        constexpr bool kRemoval = decltype(removal)::value, kSSIM = decltype(ssim)::value;
-        launch_pdl(fused_gradients_pre_kernel<PreparedSites, kRemoval, kSSIM>, grid, dim3(256),
-                   sizeof(typename GradLayout<kRemoval>::Pre), st, p, PreparedSites{geom, color});
+    with_constant(p.compute_removal != 0, [&](auto removal) {
+        with_constant(p.ssim_weight > 0.0f, [&](auto ssim) {
+            with_constant(may_crowd, [&](auto crowded) {
+                launch_pdl(fused_gradients_pre_kernel<PreparedSites, removal, ssim, crowded>, grid, dim3(256),
+                           sizeof(typename GradLayout<removal>::Pre), st, p, PreparedSites{geom, color});
+            });
+        });
     });
-}
-
-template <bool kRemoval, bool kSSIM>
-static void launch_batch_variant(const BatchArgs<GradBatchItem>& a, uint32_t tiles, cudaStream_t st) {
-    launch_pdl(fused_gradients_batch_kernel<PreparedSites, kRemoval, kSSIM>, dim3(tiles), dim3(256),
-               sizeof(typename GradLayout<kRemoval>::Pre), st, a);
+    note_launches(1);
 }
 
 void launch_gradients_batch(const GradBatchItem* items, const uint32_t* tile_prefix, uint32_t n_items,
-                            bool removal, bool ssim, cudaStream_t st) {
+                            bool removal, bool ssim, bool may_crowd, cudaStream_t st) {
     ensure_gradient_kernels();
     for_each_batch_launch(items, tile_prefix, n_items, [&](const BatchArgs<GradBatchItem>& a, uint32_t tiles) {
-        if (removal && ssim)
-            launch_batch_variant<true, true>(a, tiles, st);
-        else if (removal)
-            launch_batch_variant<true, false>(a, tiles, st);
-        else if (ssim)
-            launch_batch_variant<false, true>(a, tiles, st);
-        else
-            launch_batch_variant<false, false>(a, tiles, st);
+        with_constant(removal, [&](auto rem) {
+            with_constant(ssim, [&](auto sim) {
+                with_constant(may_crowd, [&](auto crowded) {
+                    launch_pdl(fused_gradients_batch_kernel<PreparedSites, rem, sim, crowded>, dim3(tiles), dim3(256),
+                               sizeof(typename GradLayout<rem>::Pre), st, a);
+                });
+            });
+        });
         note_launches(1);
     });
 }
@@ -699,7 +743,7 @@ extern "C" sad_status_t sad_compute_gradients_fixed(
     p += a256(size_t(site_count) * sizeof(SiteColor));
     TileMap map = tile_map_at(reinterpret_cast<uint32_t*>(p), width, height);
     launch_prepare_sites(reinterpret_cast<const Site*>(sites), geom, color, site_count, st);
-    launch_register_tiles(cand0, cand1, site_count, width, height, cand_width, cand_height, map, st);
+    launch_register_tiles(cand0, cand1, site_count, width, height, cand_width, cand_height, map, true, st);
     GradParams g{};
     g.cand0 = cand0;
     g.cand1 = cand1;
@@ -719,6 +763,6 @@ extern "C" sad_status_t sad_compute_gradients_fixed(
     g.slot_map = map.slot_map;
     g.tile_keys = map.tile_keys;
     g.tile_count = map.tile_count;
-    launch_gradients_prepared(g, geom, color, st);
+    launch_gradients_prepared(g, geom, color, true, st);
     return check_launch("sad_compute_gradients_fixed");
 }

@@ -148,10 +148,9 @@ struct GradParams {
     float removal_fix_mul;  // fixed-point path: removal delta pre-scale (a power of two, may exceed 1)
     int compute_removal;
     // trainer: the candidate field's tile registration, computed once per field refresh
-    // (nullptr: register keys inside the gradient kernel)
     const uint4* slot_map;     // [H*W] 8 x u16 tile-table index per candidate, 0xFFFF none
     const uint32_t* tile_keys;  // [tiles][kTileKeys] keys by table index
-    const int* tile_count;      // [tiles] keys in use | kTileWideFlag for a wide word table
+    const int* tile_count;      // [tiles] keys in use | kTileWideFlag for a wide word table, or kTileCrowded
 };
 struct TileMap {
     uint4* slot_map;
@@ -177,18 +176,18 @@ struct RegisterBatchItem {
     int tiles_x;
 };
 void launch_gradients_batch(const GradBatchItem* items, const uint32_t* tile_prefix, uint32_t n_items,
-                            bool removal, bool ssim, cudaStream_t st);
+                            bool removal, bool ssim, bool may_crowd, cudaStream_t st);
 void launch_register_tiles_batch(const RegisterBatchItem* items, const uint32_t* tile_prefix, uint32_t n_items,
-                                 cudaStream_t st);
+                                 bool may_crowd, cudaStream_t st);
 size_t tile_map_words(int w, int h);  // u32 words of one TileMap (slot map + keys + counts)
 TileMap tile_map_at(uint32_t* base, int w, int h);
 void launch_register_tiles(const uint32_t* c0, const uint32_t* c1, uint32_t n, int w, int h,
-                           int cw, int ch, const TileMap& map, cudaStream_t st);
+                           int cw, int ch, const TileMap& map, bool may_crowd, cudaStream_t st);
 void launch_gradients_raw(const GradParams& p, const Site* sites, cudaStream_t st);
 // Opts the >48 KB shared-memory variants in; call once per device before any capture.
 cudaError_t prepare_gradient_kernels();
 void launch_gradients_prepared(const GradParams& p, const SiteGeom* geom, const SiteColor* color,
-                               cudaStream_t st);
+                               bool may_crowd, cudaStream_t st);
 
 // optim.cu
 void launch_tau_diffuse_raw(const uint32_t* c0, const uint32_t* c1, const Site* sites,

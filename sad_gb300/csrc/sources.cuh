@@ -55,42 +55,46 @@ struct PackedSites {
 
 // Per-candidate parameter gradients for dL/dpred; out in site order.  clamp_l1 selects
 // the fused kernel's l2 = 1 / max(l1, 1e-8) (gradients.cu:383) over 1 / l1
-// (sad_bindings.cu:166).
+// (sad_bindings.cu:166).  Every operation is written with its rounding: left to the compiler,
+// which of two products a sum fuses depends on the code around it, and a fit's sums would
+// depend on which of the gradient kernel's loops a tile takes.
 __device__ __forceinline__ void candidate_grads(const SiteGeom& g, float3 col, float ux, float uy,
                                                 float inv_s2, float inv_scale, float w,
                                                 float3 dLdp, float3 pred, bool clamp_l1,
                                                 float (&o)[10]) {
-    o[4] = w * dLdp.x;
-    o[5] = w * dLdp.y;
-    o[6] = w * dLdp.z;
-    float dlogit = dLdp.x * w * (col.x - pred.x) + dLdp.y * w * (col.y - pred.y) +
-                   dLdp.z * w * (col.z - pred.z);
-    float tau = g.tau;
-    float dx = ux - g.px, dy = uy - g.py;
-    float diff2 = dx * dx + dy * dy;
-    float proj = g.dx * dx + g.dy * dy;
-    float proj2 = proj * proj;
-    float perp2 = fmaxf(diff2 - proj2, 0.0f);
-    float l1 = g.l1;
-    float l2 = (clamp_l1 && !(l1 >= 1e-8f)) ? 1.0f / 1e-8f : g.l2;
-    float d2n = (l1 * proj2 + l2 * perp2) * inv_s2;
-    float d2s = fmaxf(d2n, 1e-8f);
-    float isq = rsqrtf(d2s);
-    float rn = g.radius * inv_scale;
-    float dm = d2s * isq - rn;  // sqrt(d2s) from the reciprocal root already at hand
-    float gdx = l2 * dx + (l1 - l2) * g.dx * proj;
-    float gdy = l2 * dy + (l1 - l2) * g.dy * proj;
-    float kpos = tau * inv_s2 * isq;
-    o[0] = dlogit * kpos * gdx;
-    o[1] = dlogit * kpos * gdy;
-    o[2] = dlogit * (-dm) * tau;
-    o[3] = dlogit * tau * inv_scale;
-    float dla = (l1 * proj2 - l2 * perp2) * inv_s2;
-    float kang = dlogit * (-tau) * (0.5f * isq);
-    float kdir = 2.0f * (l1 - l2) * proj * inv_s2;
-    o[7] = kang * (kdir * dx);
-    o[8] = kang * (kdir * dy);
-    o[9] = kang * dla;
+    o[4] = __fmul_rn(w, dLdp.x);
+    o[5] = __fmul_rn(w, dLdp.y);
+    o[6] = __fmul_rn(w, dLdp.z);
+    const float dlogit = __fmaf_rn(o[6], __fsub_rn(col.z, pred.z),
+                                   __fmaf_rn(o[4], __fsub_rn(col.x, pred.x),
+                                             __fmul_rn(o[5], __fsub_rn(col.y, pred.y))));
+    const float tau = g.tau;
+    const float dx = __fsub_rn(ux, g.px), dy = __fsub_rn(uy, g.py);
+    const float diff2 = __fmaf_rn(dy, dy, __fmul_rn(dx, dx));
+    const float proj = __fmaf_rn(g.dy, dy, __fmul_rn(g.dx, dx));
+    const float proj2 = __fmul_rn(proj, proj);
+    const float perp2 = fmaxf(__fsub_rn(diff2, proj2), 0.0f);
+    const float l1 = g.l1;
+    const float l2 = (clamp_l1 && !(l1 >= 1e-8f)) ? 1.0f / 1e-8f : g.l2;
+    const float across = __fmul_rn(l2, perp2);
+    const float d2s = fmaxf(__fmul_rn(__fmaf_rn(l1, proj2, across), inv_s2), 1e-8f);
+    const float isq = rsqrtf(d2s);
+    // sqrt(d2s) from the reciprocal root already at hand
+    const float dm = __fmaf_rn(d2s, isq, -__fmul_rn(g.radius, inv_scale));
+    const float axes = __fsub_rn(l1, l2);
+    const float gdx = __fmaf_rn(l2, dx, __fmul_rn(__fmul_rn(axes, g.dx), proj));
+    const float gdy = __fmaf_rn(l2, dy, __fmul_rn(__fmul_rn(axes, g.dy), proj));
+    const float kpos = __fmul_rn(dlogit, __fmul_rn(__fmul_rn(tau, inv_s2), isq));
+    o[0] = __fmul_rn(kpos, gdx);
+    o[1] = __fmul_rn(kpos, gdy);
+    o[2] = __fmul_rn(__fmul_rn(dlogit, -dm), tau);
+    o[3] = __fmul_rn(__fmul_rn(dlogit, tau), inv_scale);
+    const float dla = __fmul_rn(__fmaf_rn(l1, proj2, -across), inv_s2);
+    const float kang = __fmul_rn(__fmul_rn(dlogit, -tau), __fmul_rn(0.5f, isq));
+    const float kdir = __fmul_rn(__fmul_rn(__fmul_rn(2.0f, axes), proj), inv_s2);
+    o[7] = __fmul_rn(kang, __fmul_rn(kdir, dx));
+    o[8] = __fmul_rn(kang, __fmul_rn(kdir, dy));
+    o[9] = __fmul_rn(kang, dla);
 }
 
 }  // namespace sad

@@ -50,21 +50,26 @@ struct SlabCarver {
 };
 
 static void drop_graphs(sad_trainer* t) {
-    for (auto& a : t->graphs)
-        for (auto& b : a)
-            for (auto& g : b)
-                if (g) {
-                    cudaGraphExecDestroy(g);
-                    g = nullptr;
-                }
-    for (auto& g : t->wgraphs)
-        if (g) {
-            cudaGraphExecDestroy(g);
-            g = nullptr;
-        }
+    auto drop = [](cudaGraphExec_t& g) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    };
+    for (auto& stage : t->graphs)
+        for (auto& upd : stage)
+            for (auto& prune : upd)
+                for (auto& g : prune) drop(g);
+    for (auto& stage : t->wgraphs)
+        for (auto& g : stage) drop(g);
 }
 
 // Host plan of the whole schedule (the same decisions the reference makes at run time).
+// The refreshes whose fields may have crowded tiles (kTileCrowded): the first ones after the
+// random lists (a 1024x1024 fit's tiles name 1,400, 1,220, 1,070, 770, 470 and 260 sites after
+// 1-6 refreshes, 84 from the tenth on), and those with most pixels holding a site of their own.
+// Later ones run kernels without that path: it costs every tile 3-4%.
+constexpr int kCrowdedRefreshes = 6;
+constexpr double kCrowdedDensity = 0.75;
+
 static void make_plan(sad_trainer* t) {
     const sad_train_config_t& c = t->cfg;
     t->plan.assign(std::max(0, c.iterations), IterPlan{});
@@ -74,8 +79,12 @@ static void make_plan(sad_trainer* t) {
     int eff_prune_end = c.prune_end > 0 ? c.prune_end : c.iterations - 1;
     int active = t->active;
     uint32_t n = t->n;
+    const int freq = c.cand_update_freq;
+    t->crowd_end = freq > 0 ? kCrowdedRefreshes * freq : c.iterations + 1;  // without refreshes: always
     for (int it = 0; it < c.iterations; ++it) {
         IterPlan& p = t->plan[it];
+        if (freq > 0 && it % freq == 0 && active > kCrowdedDensity * (static_cast<double>(t->w) * t->h))
+            t->crowd_end = std::max(t->crowd_end, it + freq);
         p.upd = c.cand_update_freq > 0 && it % c.cand_update_freq == 0;
         int desired = std::max(0, static_cast<int>(active * t->densify_pct));
         bool dens = c.densify && it >= c.densify_start && it <= c.densify_end &&
@@ -171,7 +180,8 @@ static int launch_refresh(sad_trainer* t, int src, cudaStream_t s) {
     // the new field's tile registration (a separate pass measured faster than registering
     // inside the VPT kernel, whose 32x8 blocks suit the gathers better)
     if (t->passes > 0)
-        launch_register_tiles(t->cand0[in], t->cand1[in], t->n, t->w, t->h, t->cw, t->ch, t->tmap[in], s);
+        launch_register_tiles(t->cand0[in], t->cand1[in], t->n, t->w, t->h, t->cw, t->ch, t->tmap[in],
+                              t->stage == 0, s);
     return in;
 }
 
@@ -209,7 +219,7 @@ static void launch_gradients_step(sad_trainer* t, int field, bool prune, cudaStr
     g.tile_count = t->tmap[field].tile_count;
     g.removal_fix_mul = t->removal_mul;
     g.compute_removal = prune ? 1 : 0;
-    launch_gradients_prepared(g, t->geom, t->color, s);
+    launch_gradients_prepared(g, t->geom, t->color, t->stage < 2, s);
 }
 
 // Steps 3-6 of one iteration (and the fork/join of step 1 when `upd`), then the counter
@@ -654,8 +664,8 @@ extern "C" sad_status_t sad_trainer_init(sad_trainer_t* t, const float* sites_ho
     t->alive_hint = alive_grid_hint(t);
     launch_init_candidates(t->cand0[0], t->cand1[0], n0, 0u, t->cfg.init_per_pixel ? 1 : 0, t->cw, t->ch, s);
     launch_jfa_seed(t->cand0[0], t->sites, n0, t->cw, t->ch, t->ds, s);
-    launch_register_tiles(t->cand0[0], t->cand1[0], n0, t->w, t->h, t->cw, t->ch, t->tmap[0], s);
     make_plan(t);
+    launch_register_tiles(t->cand0[0], t->cand1[0], n0, t->w, t->h, t->cw, t->ch, t->tmap[0], t->crowd_end > 0, s);
     std::vector<uint32_t> pk(std::max(1, t->cfg.iterations), 0u);
     for (size_t i = 0; i < t->plan.size(); ++i) pk[i] = t->plan[i].prune_k;
     SAD_TRY(check_cuda(cudaMemcpyAsync(t->prune_k, pk.data(), pk.size() * 4, cudaMemcpyHostToDevice, s),
@@ -694,10 +704,11 @@ extern "C" sad_status_t sad_trainer_run(sad_trainer_t* t, int end) {
     } end_run{t->tuner};
     for (int it = t->iter; it < end; ++it) {
         const IterPlan& p = t->plan[it];
+        t->stage = crowd_stage(t->crowd_end, std::max(1, c.cand_update_freq), it);
         if (!eager && window_at(t, it, end)) {
             if (use_h && (!t->hilbert_ready || t->hilbert_count != t->n)) SAD_TRY(build_hilbert(t, t->st));
-            cudaGraphExec_t& g = t->wgraphs[t->cur];
-            uint64_t& nk = t->wgraph_kernels[t->cur];
+            cudaGraphExec_t& g = t->wgraphs[t->stage][t->cur];
+            uint64_t& nk = t->wgraph_kernels[t->stage][t->cur];
             if (!g) SAD_TRY(capture_window(t, t->cur, &g, &nk));
             SAD_TRY(check_cuda(cudaGraphLaunch(g, t->st), "trainer graph launch"));
             note_launches(nk);
@@ -718,8 +729,8 @@ extern "C" sad_status_t sad_trainer_run(sad_trainer_t* t, int end) {
         } else if (eager) {
             t->cur = iteration_body(t, p.upd, p.prune, t->cur, p.upd ? t->passes : 0, t->st);
         } else {
-            cudaGraphExec_t& g = t->graphs[p.upd][p.prune][t->cur];
-            uint64_t& nk = t->graph_kernels[p.upd][p.prune][t->cur];
+            cudaGraphExec_t& g = t->graphs[t->stage][p.upd][p.prune][t->cur];
+            uint64_t& nk = t->graph_kernels[t->stage][p.upd][p.prune][t->cur];
             if (!g) SAD_TRY(capture_variant(t, p.upd, p.prune, t->cur, &g, &nk));
             SAD_TRY(check_cuda(cudaGraphLaunch(g, t->st), "trainer graph launch"));
             note_launches(nk);

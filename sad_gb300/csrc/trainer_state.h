@@ -36,6 +36,8 @@ struct sad_trainer {
     float mask_sum = 0.0f;
     uint32_t pow2 = 1, stages = 0;
     std::vector<sad::IterPlan> plan;
+    int crowd_end = 0;  // refreshes before this iteration may mark tiles as crowded
+    int stage = 0;      // crowd_stage() of the iteration being launched
 
     float* target = nullptr;
     float* mask = nullptr;
@@ -83,13 +85,14 @@ struct sad_trainer {
 
     cudaStream_t st = nullptr, side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    cudaGraphExec_t graphs[2][2][3] = {};
-    uint64_t graph_kernels[2][2][3] = {};  // kernel launches one replay runs
+    // by crowd_stage(), then refresh or not, prune or not, start field
+    cudaGraphExec_t graphs[3][2][2][3] = {};
+    uint64_t graph_kernels[3][2][2][3] = {};  // kernel launches one replay runs
     // a whole refresh window (a refresh iteration and the iterations up to the next one, no
     // densify or prune step) per start field: one replay, and programmatic dependent launch
     // across its iteration boundaries
-    cudaGraphExec_t wgraphs[3] = {};
-    uint64_t wgraph_kernels[3] = {};
+    cudaGraphExec_t wgraphs[3][3] = {};
+    uint64_t wgraph_kernels[3][3] = {};
     bool timing = false;
     std::vector<cudaEvent_t> tev;
     size_t tev_used = 0;
@@ -104,5 +107,8 @@ namespace sad {
 // order build and the VPT parameters of a trainer.
 int refresh_target_field(int passes, int src);
 sad_status_t trainer_build_hilbert(sad_trainer* t, cudaStream_t s);
+// Where iteration `it` stands: 0, its refresh may mark tiles as crowded; 1, not any more, but
+// its gradients may still read a field that has such tiles; 2, neither.
+inline int crowd_stage(int crowd_end, int freq, int it) { return it < crowd_end ? 0 : it < crowd_end + freq ? 1 : 2; }
 VptParams trainer_vpt_params(sad_trainer* t);
 }  // namespace sad
