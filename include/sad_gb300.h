@@ -125,6 +125,22 @@ sad_status_t sad_update_candidates(const uint32_t* in_cand0, const uint32_t* in_
                                    uint32_t hilbert_window, int cand_downscale, int target_width,
                                    int target_height, int width, int height, sad_stream_t stream);
 
+/* The same pass with scratch of sad_update_candidates_scratch_bytes() bytes, where each
+ * site's metric record is built once instead of at every visit.  Sites come packed, or
+ * (sites != NULL) as [n,10] f32, which the call rounds to f16 itself. */
+size_t sad_update_candidates_scratch_bytes(uint32_t site_count);
+sad_status_t sad_update_candidates_in(const uint32_t* in_cand0, const uint32_t* in_cand1,
+                                      uint32_t* out_cand0, uint32_t* out_cand1,
+                                      const uint16_t* packed_sites, const float* sites,
+                                      uint32_t site_count, uint32_t step, float inv_scale_sq,
+                                      uint32_t step_high, float radius_scale,
+                                      uint32_t radius_probes, uint32_t inject_count,
+                                      const uint32_t* hilbert_order, const uint32_t* hilbert_pos,
+                                      uint32_t hilbert_probes, uint32_t hilbert_window,
+                                      int cand_downscale, int target_width, int target_height,
+                                      int width, int height, void* scratch, size_t scratch_bytes,
+                                      sad_stream_t stream);
+
 /* Jump step of the VPT schedule: pow2(maxdim) >> (min(i, stages-1) + 1), and its packed
  * form (jump << 16) | (i & 0xffff).
  * replaces: jumpStepForIndex / packJumpStep, backends/cuda/src/sad_cuda.cu:1157-1183 */

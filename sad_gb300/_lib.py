@@ -81,6 +81,9 @@ SIGNATURES = {
     "sad_jfa_flood": (st, [vp, vp, vp, u32, u32, f32, i32, i32, i32, i32, i32, vp]),
     "sad_update_candidates": (st, [vp, vp, vp, vp, vp, u32, u32, f32, u32, f32, u32, u32, vp, vp,
                                    u32, u32, i32, i32, i32, i32, i32, vp]),
+    "sad_update_candidates_scratch_bytes": (sz, [u32]),
+    "sad_update_candidates_in": (st, [vp, vp, vp, vp, vp, vp, u32, u32, f32, u32, f32, u32, u32, vp, vp,
+                                      u32, u32, i32, i32, i32, i32, i32, vp, sz, vp]),
     "sad_jump_step_for_index": (u32, [u32, i32, i32]),
     "sad_pack_jump_step": (u32, [u32, i32, i32]),
     "sad_compute_gradients_tiled": (st, [vp, vp, vp, vp, vp] + [vp] * 10 +

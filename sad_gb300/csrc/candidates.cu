@@ -140,6 +140,18 @@ void launch_pack_geom_alive(const Site* sites, SiteGeom* out, const uint32_t* al
     note_launches(1);
 }
 
+// The records of packed sites, once per site and call instead of once per visit.
+__global__ void unpack_geom_kernel(const uint4* __restrict__ packed, SiteGeom* __restrict__ out, uint32_t n) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) store_geom(out, i, geom_from_packed(packed[i]));
+}
+
+static void launch_unpack_geom(const uint16_t* packed, SiteGeom* out, uint32_t n, cudaStream_t st) {
+    if (n == 0) return;
+    unpack_geom_kernel<<<blocks_for(n, 256), 256, 0, st>>>(reinterpret_cast<const uint4*>(packed), out, n);
+    note_launches(1);
+}
+
 struct PackedHalfSites {
     const uint4* p;
     __device__ __forceinline__ SiteGeom load(uint32_t id) const { return geom_from_packed(__ldg(p + id)); }
@@ -766,20 +778,21 @@ extern "C" sad_status_t sad_jfa_flood(const uint32_t* in_cand0, uint32_t* out_ca
     return check_launch("sad_jfa_flood");
 }
 
-extern "C" sad_status_t sad_update_candidates(
+// sites: raw sites (nullptr: packed_sites); records: scratch for a record per site (nullptr:
+// the pass decodes packed_sites at every visit).
+static sad_status_t update_candidates(
     const uint32_t* in_cand0, const uint32_t* in_cand1, uint32_t* out_cand0, uint32_t* out_cand1,
-    const uint16_t* packed_sites, uint32_t site_count, uint32_t step, float inv_scale_sq,
+    const uint16_t* packed_sites, const float* sites, uint32_t site_count, uint32_t step, float inv_scale_sq,
     uint32_t step_high, float radius_scale, uint32_t radius_probes, uint32_t inject_count,
     const uint32_t* hilbert_order, const uint32_t* hilbert_pos, uint32_t hilbert_probes,
     uint32_t hilbert_window, int cand_downscale, int target_width, int target_height, int width,
-    int height, sad_stream_t stream) {
-    clear_error();
+    int height, SiteGeom* records, cudaStream_t stream) {
     SAD_REQUIRE(image_size_ok(width, height), "sad_update_candidates: invalid cand size");
     SAD_REQUIRE(target_width > 0 && target_height > 0, "sad_update_candidates: invalid target size");
     SAD_REQUIRE(in_cand0 && in_cand1 && out_cand0 && out_cand1, "sad_update_candidates: null field");
     SAD_REQUIRE(in_cand0 != out_cand0 && in_cand1 != out_cand1,
                 "sad_update_candidates: in and out fields must differ");
-    SAD_REQUIRE(site_count == 0 || packed_sites, "sad_update_candidates: null packed sites");
+    SAD_REQUIRE(site_count == 0 || packed_sites || sites, "sad_update_candidates: null packed sites");
     bool use_h = hilbert_probes > 0 && hilbert_window > 0;
     SAD_REQUIRE(!use_h || (hilbert_order && hilbert_pos),
                 "sad_update_candidates: hilbert probes need hilbert_order and hilbert_pos");
@@ -805,6 +818,49 @@ extern "C" sad_status_t sad_update_candidates(
     prm.width = width;
     prm.height = height;
     prm.state = nullptr;
-    launch_vpt_packed(prm, packed_sites, as_stream(stream));
+    if (!records) {
+        launch_vpt_packed(prm, packed_sites, stream);
+    } else {
+        if (sites)
+            launch_pack_geom(reinterpret_cast<const Site*>(sites), records, site_count, stream);
+        else
+            launch_unpack_geom(packed_sites, records, site_count, stream);
+        launch_vpt_geom(prm, records, stream);
+    }
     return check_launch("sad_update_candidates");
+}
+
+extern "C" sad_status_t sad_update_candidates(
+    const uint32_t* in_cand0, const uint32_t* in_cand1, uint32_t* out_cand0, uint32_t* out_cand1,
+    const uint16_t* packed_sites, uint32_t site_count, uint32_t step, float inv_scale_sq,
+    uint32_t step_high, float radius_scale, uint32_t radius_probes, uint32_t inject_count,
+    const uint32_t* hilbert_order, const uint32_t* hilbert_pos, uint32_t hilbert_probes,
+    uint32_t hilbert_window, int cand_downscale, int target_width, int target_height, int width,
+    int height, sad_stream_t stream) {
+    clear_error();
+    return update_candidates(in_cand0, in_cand1, out_cand0, out_cand1, packed_sites, nullptr, site_count, step,
+                             inv_scale_sq, step_high, radius_scale, radius_probes, inject_count, hilbert_order,
+                             hilbert_pos, hilbert_probes, hilbert_window, cand_downscale, target_width,
+                             target_height, width, height, nullptr, as_stream(stream));
+}
+
+extern "C" size_t sad_update_candidates_scratch_bytes(uint32_t site_count) {
+    return static_cast<size_t>(site_count) * sizeof(SiteGeom) + alignof(SiteGeom);
+}
+
+extern "C" sad_status_t sad_update_candidates_in(
+    const uint32_t* in_cand0, const uint32_t* in_cand1, uint32_t* out_cand0, uint32_t* out_cand1,
+    const uint16_t* packed_sites, const float* sites, uint32_t site_count, uint32_t step, float inv_scale_sq,
+    uint32_t step_high, float radius_scale, uint32_t radius_probes, uint32_t inject_count,
+    const uint32_t* hilbert_order, const uint32_t* hilbert_pos, uint32_t hilbert_probes,
+    uint32_t hilbert_window, int cand_downscale, int target_width, int target_height, int width,
+    int height, void* scratch, size_t scratch_bytes, sad_stream_t stream) {
+    clear_error();
+    SAD_REQUIRE(scratch && scratch_bytes >= sad_update_candidates_scratch_bytes(site_count),
+                "sad_update_candidates_in: scratch too small");
+    const uintptr_t base = (reinterpret_cast<uintptr_t>(scratch) + alignof(SiteGeom) - 1) & ~(alignof(SiteGeom) - 1);
+    return update_candidates(in_cand0, in_cand1, out_cand0, out_cand1, packed_sites, sites, site_count, step,
+                             inv_scale_sq, step_high, radius_scale, radius_probes, inject_count, hilbert_order,
+                             hilbert_pos, hilbert_probes, hilbert_window, cand_downscale, target_width,
+                             target_height, width, height, reinterpret_cast<SiteGeom*>(base), as_stream(stream));
 }

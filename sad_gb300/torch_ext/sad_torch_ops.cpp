@@ -59,6 +59,10 @@ T* ptr(const Tensor& t) {
 
 uint32_t u32(int64_t v) { return static_cast<uint32_t>(v); }
 
+Tensor scratch_for(const Tensor& like, size_t bytes) {
+    return at::empty({static_cast<int64_t>(bytes)}, like.options().dtype(at::kByte));
+}
+
 // ---------------------------------------------------------------------------
 // render / adjoint / candidates
 // ---------------------------------------------------------------------------
@@ -106,7 +110,7 @@ std::tuple<Tensor, Tensor> init_candidates(int64_t width, int64_t height, int64_
     return {cand0, cand1};
 }
 
-// sad_bindings.cu:623-696 (vptPass): packs the sites to f16 and runs one pass with
+// sad_bindings.cu:623-696 (vptPass): rounds the sites to f16 and runs one pass with
 // step = jump << 16 and no Hilbert probes; `seed` is unused, as in the reference.
 std::tuple<Tensor, Tensor> vpt_pass(const Tensor& cand0_, const Tensor& cand1_, const Tensor& sites_,
                                     double inv_scale_sq, int64_t width, int64_t height, int64_t jump,
@@ -120,15 +124,14 @@ std::tuple<Tensor, Tensor> vpt_pass(const Tensor& cand0_, const Tensor& cand1_, 
     c10::cuda::CUDAGuard guard(cand0_.device());
     Tensor cand0 = cand0_.contiguous(), cand1 = cand1_.contiguous(), sites = sites_.contiguous();
     Tensor out0 = at::empty_like(cand0), out1 = at::empty_like(cand1);
-    Tensor packed = at::empty({sites.size(0), 8}, sites.options().dtype(at::kHalf));
-    sad_stream_t s = stream_of(cand0);
-    ok(sad_pack_candidate_sites(ptr(sites), ptr<uint16_t>(packed), u32(sites.size(0)), s));
-    ok(sad_update_candidates(ptr<uint32_t>(cand0), ptr<uint32_t>(cand1), ptr<uint32_t>(out0), ptr<uint32_t>(out1),
-                             ptr<uint16_t>(packed), u32(sites.size(0)), u32(jump << 16),
-                             static_cast<float>(inv_scale_sq), 0u, static_cast<float>(radius_scale),
-                             u32(radius_probes), u32(inject_count), nullptr, nullptr, 0u, 0u, 1,
-                             static_cast<int>(width), static_cast<int>(height), static_cast<int>(width),
-                             static_cast<int>(height), s));
+    Tensor scratch = scratch_for(sites, sad_update_candidates_scratch_bytes(u32(sites.size(0))));
+    ok(sad_update_candidates_in(ptr<uint32_t>(cand0), ptr<uint32_t>(cand1), ptr<uint32_t>(out0), ptr<uint32_t>(out1),
+                                nullptr, ptr(sites), u32(sites.size(0)), u32(jump << 16),
+                                static_cast<float>(inv_scale_sq), 0u, static_cast<float>(radius_scale),
+                                u32(radius_probes), u32(inject_count), nullptr, nullptr, 0u, 0u, 1,
+                                static_cast<int>(width), static_cast<int>(height), static_cast<int>(width),
+                                static_cast<int>(height), scratch.data_ptr(), static_cast<size_t>(scratch.numel()),
+                                stream_of(cand0)));
     return {out0, out1};
 }
 
@@ -179,6 +182,8 @@ Tensor pack_candidate_sites(const Tensor& sites_, const Tensor& packed_, int64_t
     return packed;
 }
 
+constexpr int64_t kRecordTexels = 1 << 17;
+
 // sad_bindings.cu:786-863
 Tensor update_candidates_compact(const Tensor& cand0_in_, const Tensor& cand1_in_, const Tensor& cand0_out_,
                                  const Tensor& cand1_out_, const Tensor& packed_sites_, const Tensor& hilbert_order,
@@ -210,6 +215,19 @@ Tensor update_candidates_compact(const Tensor& cand0_in_, const Tensor& cand1_in
         hp = hilbert_pos.contiguous();
         hop = ptr<uint32_t>(ho);
         hpp = ptr<uint32_t>(hp);
+    }
+    // decoding each site once costs a launch: on fields it does not pay for, the pass decodes
+    if (cand_width * cand_height >= kRecordTexels && site_count <= cand_width * cand_height) {
+        Tensor scratch = scratch_for(packed_sites, sad_update_candidates_scratch_bytes(u32(site_count)));
+        ok(sad_update_candidates_in(
+            ptr<uint32_t>(cand0_in), ptr<uint32_t>(cand1_in), ptr<uint32_t>(cand0_out), ptr<uint32_t>(cand1_out),
+            ptr<uint16_t>(packed_sites), nullptr, u32(site_count), u32(step), static_cast<float>(inv_scale_sq),
+            u32(step_high), static_cast<float>(radius_scale), u32(radius_probes), u32(inject_count), hop, hpp,
+            u32(hilbert_probes), u32(hilbert_window), static_cast<int>(cand_downscale),
+            static_cast<int>(target_width), static_cast<int>(target_height), static_cast<int>(cand_width),
+            static_cast<int>(cand_height), scratch.data_ptr(), static_cast<size_t>(scratch.numel()),
+            stream_of(cand0_in)));
+        return cand0_out;
     }
     ok(sad_update_candidates(ptr<uint32_t>(cand0_in), ptr<uint32_t>(cand1_in), ptr<uint32_t>(cand0_out),
                              ptr<uint32_t>(cand1_out), ptr<uint16_t>(packed_sites), u32(site_count), u32(step),
