@@ -70,6 +70,15 @@ sad_status_t sad_render(const uint32_t* cand0, const uint32_t* cand1, float* out
                         const float* sites, float inv_scale_sq, uint32_t site_count, int width,
                         int height, int cand_width, int cand_height, sad_stream_t stream);
 
+/* The same with scratch of sad_site_scratch_bytes() bytes, where each site's metric record is
+ * built once instead of at every visit.  So also sad_render_backward_in and
+ * sad_compute_gradients_tiled_in below. */
+size_t sad_site_scratch_bytes(uint32_t site_count);
+sad_status_t sad_render_in(const uint32_t* cand0, const uint32_t* cand1, float* out_rgb,
+                           const float* sites, float inv_scale_sq, uint32_t site_count, int width,
+                           int height, int cand_width, int cand_height, void* scratch,
+                           size_t scratch_bytes, sad_stream_t stream);
+
 /* Adjoint of sad_render: dL/dsites [N,10] ACCUMULATED into grad_sites (zero it first).
  * Softmax weights are recomputed, nothing is stored by the forward.
  * replaces: render_sad_backward_kernel, backends/pytorch/torch_ext/cuda/sad_bindings.cu:100-207
@@ -78,6 +87,12 @@ sad_status_t sad_render_backward(const uint32_t* cand0, const uint32_t* cand1,
                                  const float* grad_rgb, float* grad_sites, const float* sites,
                                  float inv_scale_sq, uint32_t site_count, int width, int height,
                                  int cand_width, int cand_height, sad_stream_t stream);
+
+sad_status_t sad_render_backward_in(const uint32_t* cand0, const uint32_t* cand1,
+                                    const float* grad_rgb, float* grad_sites, const float* sites,
+                                    float inv_scale_sq, uint32_t site_count, int width, int height,
+                                    int cand_width, int cand_height, void* scratch,
+                                    size_t scratch_bytes, sad_stream_t stream);
 
 /* Random (xorshift) or per-pixel-neighbourhood candidate init.
  * replaces: launchInitCandidates, backends/cuda/src/render.cu:181-197 */
@@ -163,6 +178,15 @@ sad_status_t sad_compute_gradients_tiled(
     float inv_scale_sq, uint32_t site_count, float* removal_delta, uint32_t compute_removal,
     float ssim_weight, int width, int height, int cand_width, int cand_height,
     sad_stream_t stream);
+
+sad_status_t sad_compute_gradients_tiled_in(
+    const uint32_t* cand0, const uint32_t* cand1, const float* target, const float* rendered,
+    const float* mask, float* grad_pos_x, float* grad_pos_y, float* grad_log_tau,
+    float* grad_radius, float* grad_color_r, float* grad_color_g, float* grad_color_b,
+    float* grad_dir_x, float* grad_dir_y, float* grad_log_aniso, const float* sites,
+    float inv_scale_sq, uint32_t site_count, float* removal_delta, uint32_t compute_removal,
+    float ssim_weight, int width, int height, int cand_width, int cand_height, void* scratch,
+    size_t scratch_bytes, sad_stream_t stream);
 
 /* The trainer's form of the same evaluation, the kernel a fit runs every iteration: the
  * candidate field's 16x16-tile registration, then per-site sums in exact 64-bit fixed

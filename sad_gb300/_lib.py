@@ -74,6 +74,9 @@ SIGNATURES = {
     "sad_launch_count": (C.c_uint64, []),
     "sad_render": (st, [vp, vp, vp, vp, f32, u32, i32, i32, i32, i32, vp]),
     "sad_render_backward": (st, [vp, vp, vp, vp, vp, f32, u32, i32, i32, i32, i32, vp]),
+    "sad_site_scratch_bytes": (sz, [u32]),
+    "sad_render_in": (st, [vp, vp, vp, vp, f32, u32, i32, i32, i32, i32, vp, sz, vp]),
+    "sad_render_backward_in": (st, [vp, vp, vp, vp, vp, f32, u32, i32, i32, i32, i32, vp, sz, vp]),
     "sad_init_candidates": (st, [vp, vp, u32, u32, i32, i32, i32, vp]),
     "sad_clear_candidates": (st, [vp, vp, i32, i32, vp]),
     "sad_pack_candidate_sites": (st, [vp, vp, u32, vp]),
@@ -88,6 +91,8 @@ SIGNATURES = {
     "sad_pack_jump_step": (u32, [u32, i32, i32]),
     "sad_compute_gradients_tiled": (st, [vp, vp, vp, vp, vp] + [vp] * 10 +
                                     [vp, f32, u32, vp, u32, f32, i32, i32, i32, i32, vp]),
+    "sad_compute_gradients_tiled_in": (st, [vp, vp, vp, vp, vp] + [vp] * 10 +
+                                       [vp, f32, u32, vp, u32, f32, i32, i32, i32, i32, vp, sz, vp]),
     "sad_compute_gradients_fixed_scratch_bytes": (sz, [u32, i32, i32]),
     "sad_compute_gradients_fixed": (st, [vp, vp, vp, vp, vp, vp, f32, u32, u32, f32, i32, i32, i32, i32,
                                          vp, vp, vp, sz, vp]),

@@ -624,11 +624,12 @@ cudaError_t prepare_gradient_kernels() {
     });
 }
 
-void launch_gradients_raw(const GradParams& p, const Site* sites, cudaStream_t st) {
+template <class Src>
+static void launch_gradients_float(const GradParams& p, Src src, cudaStream_t st) {
     const dim3 grid((p.width + 31) / 32, (p.height + 7) / 8);
     with_constant(p.compute_removal != 0, [&](auto removal) {
         with_constant(p.ssim_weight > 0.0f, [&](auto ssim) {
-            fused_gradients_kernel<RawSites, removal, ssim><<<grid, 256, 0, st>>>(p, RawSites{sites});
+            fused_gradients_kernel<Src, removal, ssim><<<grid, 256, 0, st>>>(p, src);
         });
     });
     note_launches(1);
@@ -670,15 +671,15 @@ void launch_gradients_batch(const GradBatchItem* items, const uint32_t* tile_pre
 
 using namespace sad;
 
-extern "C" sad_status_t sad_compute_gradients_tiled(
+// The gradients of the API (scratch: room for prepared site records, or nullptr).
+static sad_status_t compute_gradients_float(
     const uint32_t* cand0, const uint32_t* cand1, const float* target, const float* rendered,
     const float* mask, float* grad_pos_x, float* grad_pos_y, float* grad_log_tau,
     float* grad_radius, float* grad_color_r, float* grad_color_g, float* grad_color_b,
     float* grad_dir_x, float* grad_dir_y, float* grad_log_aniso, const float* sites,
     float inv_scale_sq, uint32_t site_count, float* removal_delta, uint32_t compute_removal,
-    float ssim_weight, int width, int height, int cand_width, int cand_height,
+    float ssim_weight, int width, int height, int cand_width, int cand_height, void* scratch,
     sad_stream_t stream) {
-    clear_error();
     SAD_REQUIRE(image_size_ok(width, height), "sad_compute_gradients_tiled: invalid image size");
     SAD_REQUIRE(image_size_ok(cand_width, cand_height), "sad_compute_gradients_tiled: invalid cand size");
     SAD_REQUIRE(cand0 && cand1 && target, "sad_compute_gradients_tiled: null input");
@@ -707,8 +708,44 @@ extern "C" sad_status_t sad_compute_gradients_tiled(
     p.removal = removal_delta;
     p.fix12 = nullptr;
     p.compute_removal = compute_removal ? 1 : 0;
-    launch_gradients_raw(p, reinterpret_cast<const Site*>(sites), as_stream(stream));
+    cudaStream_t st = as_stream(stream);
+    if (scratch)
+        launch_gradients_float(p, prepare_in_scratch(sites, site_count, scratch, st), st);
+    else
+        launch_gradients_float(p, RawSites{reinterpret_cast<const Site*>(sites)}, st);
     return check_launch("sad_compute_gradients_tiled");
+}
+
+extern "C" sad_status_t sad_compute_gradients_tiled(
+    const uint32_t* cand0, const uint32_t* cand1, const float* target, const float* rendered,
+    const float* mask, float* grad_pos_x, float* grad_pos_y, float* grad_log_tau,
+    float* grad_radius, float* grad_color_r, float* grad_color_g, float* grad_color_b,
+    float* grad_dir_x, float* grad_dir_y, float* grad_log_aniso, const float* sites,
+    float inv_scale_sq, uint32_t site_count, float* removal_delta, uint32_t compute_removal,
+    float ssim_weight, int width, int height, int cand_width, int cand_height,
+    sad_stream_t stream) {
+    clear_error();
+    return compute_gradients_float(cand0, cand1, target, rendered, mask, grad_pos_x, grad_pos_y, grad_log_tau,
+                                   grad_radius, grad_color_r, grad_color_g, grad_color_b, grad_dir_x, grad_dir_y,
+                                   grad_log_aniso, sites, inv_scale_sq, site_count, removal_delta, compute_removal,
+                                   ssim_weight, width, height, cand_width, cand_height, nullptr, stream);
+}
+
+extern "C" sad_status_t sad_compute_gradients_tiled_in(
+    const uint32_t* cand0, const uint32_t* cand1, const float* target, const float* rendered,
+    const float* mask, float* grad_pos_x, float* grad_pos_y, float* grad_log_tau,
+    float* grad_radius, float* grad_color_r, float* grad_color_g, float* grad_color_b,
+    float* grad_dir_x, float* grad_dir_y, float* grad_log_aniso, const float* sites,
+    float inv_scale_sq, uint32_t site_count, float* removal_delta, uint32_t compute_removal,
+    float ssim_weight, int width, int height, int cand_width, int cand_height, void* scratch,
+    size_t scratch_bytes, sad_stream_t stream) {
+    clear_error();
+    SAD_REQUIRE(scratch && scratch_bytes >= sad_site_scratch_bytes(site_count),
+                "sad_compute_gradients_tiled_in: scratch too small");
+    return compute_gradients_float(cand0, cand1, target, rendered, mask, grad_pos_x, grad_pos_y, grad_log_tau,
+                                   grad_radius, grad_color_r, grad_color_g, grad_color_b, grad_dir_x, grad_dir_y,
+                                   grad_log_aniso, sites, inv_scale_sq, site_count, removal_delta, compute_removal,
+                                   ssim_weight, width, height, cand_width, cand_height, scratch, stream);
 }
 
 extern "C" size_t sad_compute_gradients_fixed_scratch_bytes(uint32_t site_count, int width, int height) {

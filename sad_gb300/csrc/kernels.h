@@ -106,9 +106,6 @@ void launch_unpack_inference(const uint32_t* packed, const float* quant, uint32_
 void launch_init_candidates(uint32_t* c0, uint32_t* c1, uint32_t n, uint32_t seed, int per_pixel,
                             int w, int h, cudaStream_t st);
 void launch_clear_candidates(uint32_t* c0, uint32_t* c1, int w, int h, cudaStream_t st);
-void launch_render_backward_raw(const uint32_t* c0, const uint32_t* c1, const float* grad_rgb,
-                                float* grad_sites, const Site* sites, float inv_s2, uint32_t n,
-                                int w, int h, int cw, int ch, cudaStream_t st);
 
 // candidates.cu
 void launch_pack_sites(const Site* sites, uint16_t* packed, uint32_t n, cudaStream_t st);
@@ -183,7 +180,6 @@ size_t tile_map_words(int w, int h);  // u32 words of one TileMap (slot map + ke
 TileMap tile_map_at(uint32_t* base, int w, int h);
 void launch_register_tiles(const uint32_t* c0, const uint32_t* c1, uint32_t n, int w, int h,
                            int cw, int ch, const TileMap& map, bool may_crowd, cudaStream_t st);
-void launch_gradients_raw(const GradParams& p, const Site* sites, cudaStream_t st);
 // Opts the >48 KB shared-memory variants in; call once per device before any capture.
 cudaError_t prepare_gradient_kernels();
 void launch_gradients_prepared(const GradParams& p, const SiteGeom* geom, const SiteColor* color,

@@ -279,12 +279,13 @@ __global__ void __launch_bounds__(256, 4) render_backward_kernel(
         [&](uint32_t id, int k, float v) { atomicAdd(grad_sites + static_cast<size_t>(id) * 10 + k, v); });
 }
 
-void launch_render_backward_raw(const uint32_t* c0, const uint32_t* c1, const float* grad_rgb,
-                                float* grad_sites, const Site* sites, float inv_s2, uint32_t n,
-                                int w, int h, int cw, int ch, cudaStream_t st) {
-    render_backward_kernel<RawSites><<<pixel_grid(w, h), dim3(32, 8), 0, st>>>(
-        reinterpret_cast<const uint4*>(c0), reinterpret_cast<const uint4*>(c1), grad_rgb, grad_sites,
-        RawSites{sites}, inv_s2, n, w, h, cw, ch);
+template <class Src>
+static void launch_render_backward(const uint32_t* c0, const uint32_t* c1, const float* grad_rgb,
+                                   float* grad_sites, Src src, float inv_s2, uint32_t n,
+                                   int w, int h, int cw, int ch, cudaStream_t st) {
+    render_backward_kernel<Src><<<pixel_grid(w, h), dim3(32, 8), 0, st>>>(
+        reinterpret_cast<const uint4*>(c0), reinterpret_cast<const uint4*>(c1), grad_rgb, grad_sites, src,
+        inv_s2, n, w, h, cw, ch);
     note_launches(1);
 }
 
@@ -295,18 +296,63 @@ void launch_render_backward_raw(const uint32_t* c0, const uint32_t* c1, const fl
 // ---------------------------------------------------------------------------
 using namespace sad;
 
+static sad_status_t check_render(const uint32_t* cand0, const uint32_t* cand1, const float* out_rgb,
+                                 const float* sites, uint32_t site_count, int width, int height,
+                                 int cand_width, int cand_height) {
+    SAD_REQUIRE(image_size_ok(width, height), "sad_render: invalid image size");
+    SAD_REQUIRE(image_size_ok(cand_width, cand_height), "sad_render: invalid cand size");
+    SAD_REQUIRE(cand0 && cand1 && out_rgb, "sad_render: null buffer");
+    SAD_REQUIRE(sites || site_count == 0, "sad_render: null sites");
+    return SAD_OK;
+}
+
 extern "C" sad_status_t sad_render(const uint32_t* cand0, const uint32_t* cand1, float* out_rgb,
                                    const float* sites, float inv_scale_sq, uint32_t site_count,
                                    int width, int height, int cand_width, int cand_height,
                                    sad_stream_t stream) {
     clear_error();
-    SAD_REQUIRE(image_size_ok(width, height), "sad_render: invalid image size");
-    SAD_REQUIRE(image_size_ok(cand_width, cand_height), "sad_render: invalid cand size");
-    SAD_REQUIRE(cand0 && cand1 && out_rgb, "sad_render: null buffer");
-    SAD_REQUIRE(sites || site_count == 0, "sad_render: null sites");
+    SAD_TRY(check_render(cand0, cand1, out_rgb, sites, site_count, width, height, cand_width, cand_height));
     launch_render_raw(cand0, cand1, out_rgb, reinterpret_cast<const Site*>(sites), inv_scale_sq,
                       site_count, width, height, cand_width, cand_height, as_stream(stream));
     return check_launch("sad_render");
+}
+
+extern "C" size_t sad_site_scratch_bytes(uint32_t site_count) {
+    return static_cast<size_t>(site_count) * (sizeof(SiteGeom) + sizeof(SiteColor)) + alignof(SiteGeom);
+}
+
+namespace sad {
+PreparedSites prepare_in_scratch(const float* sites, uint32_t n, void* scratch, cudaStream_t st) {
+    const uintptr_t base = (reinterpret_cast<uintptr_t>(scratch) + alignof(SiteGeom) - 1) & ~(alignof(SiteGeom) - 1);
+    SiteGeom* geom = reinterpret_cast<SiteGeom*>(base);
+    SiteColor* color = reinterpret_cast<SiteColor*>(geom + n);
+    launch_prepare_sites(reinterpret_cast<const Site*>(sites), geom, color, n, st);
+    return PreparedSites{geom, color};
+}
+}  // namespace sad
+
+extern "C" sad_status_t sad_render_in(const uint32_t* cand0, const uint32_t* cand1, float* out_rgb,
+                                      const float* sites, float inv_scale_sq, uint32_t site_count,
+                                      int width, int height, int cand_width, int cand_height,
+                                      void* scratch, size_t scratch_bytes, sad_stream_t stream) {
+    clear_error();
+    SAD_TRY(check_render(cand0, cand1, out_rgb, sites, site_count, width, height, cand_width, cand_height));
+    SAD_REQUIRE(scratch && scratch_bytes >= sad_site_scratch_bytes(site_count), "sad_render_in: scratch too small");
+    cudaStream_t st = as_stream(stream);
+    const PreparedSites p = prepare_in_scratch(sites, site_count, scratch, st);
+    launch_render_prepared(cand0, cand1, out_rgb, p.g, p.c, inv_scale_sq, site_count, width, height, cand_width,
+                           cand_height, st);
+    return check_launch("sad_render_in");
+}
+
+static sad_status_t check_render_backward(const uint32_t* cand0, const uint32_t* cand1, const float* grad_rgb,
+                                          const float* grad_sites, const float* sites, uint32_t site_count,
+                                          int width, int height, int cand_width, int cand_height) {
+    SAD_REQUIRE(image_size_ok(width, height), "sad_render_backward: invalid image size");
+    SAD_REQUIRE(image_size_ok(cand_width, cand_height), "sad_render_backward: invalid cand size");
+    SAD_REQUIRE(cand0 && cand1 && grad_rgb && grad_sites, "sad_render_backward: null buffer");
+    SAD_REQUIRE(sites || site_count == 0, "sad_render_backward: null sites");
+    return SAD_OK;
 }
 
 extern "C" sad_status_t sad_render_backward(const uint32_t* cand0, const uint32_t* cand1,
@@ -315,14 +361,28 @@ extern "C" sad_status_t sad_render_backward(const uint32_t* cand0, const uint32_
                                             uint32_t site_count, int width, int height,
                                             int cand_width, int cand_height, sad_stream_t stream) {
     clear_error();
-    SAD_REQUIRE(image_size_ok(width, height), "sad_render_backward: invalid image size");
-    SAD_REQUIRE(image_size_ok(cand_width, cand_height), "sad_render_backward: invalid cand size");
-    SAD_REQUIRE(cand0 && cand1 && grad_rgb && grad_sites, "sad_render_backward: null buffer");
-    SAD_REQUIRE(sites || site_count == 0, "sad_render_backward: null sites");
-    launch_render_backward_raw(cand0, cand1, grad_rgb, grad_sites,
-                               reinterpret_cast<const Site*>(sites), inv_scale_sq, site_count,
-                               width, height, cand_width, cand_height, as_stream(stream));
+    SAD_TRY(check_render_backward(cand0, cand1, grad_rgb, grad_sites, sites, site_count, width, height, cand_width,
+                                  cand_height));
+    launch_render_backward(cand0, cand1, grad_rgb, grad_sites, RawSites{reinterpret_cast<const Site*>(sites)},
+                           inv_scale_sq, site_count, width, height, cand_width, cand_height, as_stream(stream));
     return check_launch("sad_render_backward");
+}
+
+extern "C" sad_status_t sad_render_backward_in(const uint32_t* cand0, const uint32_t* cand1,
+                                               const float* grad_rgb, float* grad_sites,
+                                               const float* sites, float inv_scale_sq,
+                                               uint32_t site_count, int width, int height,
+                                               int cand_width, int cand_height, void* scratch,
+                                               size_t scratch_bytes, sad_stream_t stream) {
+    clear_error();
+    SAD_TRY(check_render_backward(cand0, cand1, grad_rgb, grad_sites, sites, site_count, width, height, cand_width,
+                                  cand_height));
+    SAD_REQUIRE(scratch && scratch_bytes >= sad_site_scratch_bytes(site_count),
+                "sad_render_backward_in: scratch too small");
+    cudaStream_t st = as_stream(stream);
+    launch_render_backward(cand0, cand1, grad_rgb, grad_sites, prepare_in_scratch(sites, site_count, scratch, st),
+                           inv_scale_sq, site_count, width, height, cand_width, cand_height, st);
+    return check_launch("sad_render_backward_in");
 }
 
 extern "C" sad_status_t sad_init_candidates(uint32_t* cand0, uint32_t* cand1, uint32_t site_count,

@@ -35,6 +35,9 @@ struct PreparedSites {
     __device__ __forceinline__ void prepare() {}
 };
 
+// Prepares n raw sites in caller scratch of sad_site_scratch_bytes(n) bytes (render.cu).
+PreparedSites prepare_in_scratch(const float* sites, uint32_t n, void* scratch, cudaStream_t st);
+
 // 16-byte quantised sites (packed.cuh), decoded per candidate; an inactive site reads as
 // position (-1, -1) so it is skipped like a pruned one (packedActive,
 // backends/metal/shaders/sad_common.metal:85-87).  prepare() loads the ranges once per thread.

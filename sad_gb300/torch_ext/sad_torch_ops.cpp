@@ -59,6 +59,11 @@ T* ptr(const Tensor& t) {
 
 uint32_t u32(int64_t v) { return static_cast<uint32_t>(v); }
 
+// Whether site records, built once per call by a launch of their own, pay for themselves in a
+// kernel over `pixels` that reads eight sites each.
+constexpr int64_t kRecordPixels = 1 << 19;
+bool records_pay(int64_t pixels, int64_t sites) { return pixels >= kRecordPixels && sites <= pixels; }
+
 Tensor scratch_for(const Tensor& like, size_t bytes) {
     return at::empty({static_cast<int64_t>(bytes)}, like.options().dtype(at::kByte));
 }
@@ -80,6 +85,14 @@ Tensor render_sad_padded(const Tensor& cand0_, const Tensor& cand1_, const Tenso
     c10::cuda::CUDAGuard guard(cand0_.device());
     Tensor cand0 = cand0_.contiguous(), cand1 = cand1_.contiguous(), sites = sites_.contiguous();
     Tensor out = at::empty({height, width, 3}, cand0.options().dtype(at::kFloat));
+    if (records_pay(width * height, sites.size(0))) {
+        Tensor scratch = scratch_for(sites, sad_site_scratch_bytes(u32(sites.size(0))));
+        ok(sad_render_in(ptr<uint32_t>(cand0), ptr<uint32_t>(cand1), ptr(out), ptr(sites),
+                         static_cast<float>(inv_scale_sq), u32(sites.size(0)), static_cast<int>(width),
+                         static_cast<int>(height), static_cast<int>(cand_width), static_cast<int>(cand_height),
+                         scratch.data_ptr(), static_cast<size_t>(scratch.numel()), stream_of(cand0)));
+        return out;
+    }
     ok(sad_render(ptr<uint32_t>(cand0), ptr<uint32_t>(cand1), ptr(out), ptr(sites), static_cast<float>(inv_scale_sq),
                   u32(sites.size(0)), static_cast<int>(width), static_cast<int>(height),
                   static_cast<int>(cand_width), static_cast<int>(cand_height), stream_of(cand0)));
@@ -151,6 +164,15 @@ Tensor render_sad_backward(const Tensor& cand0_, const Tensor& cand1_, const Ten
     Tensor cand0 = cand0_.contiguous(), cand1 = cand1_.contiguous();
     Tensor sites = sites_.contiguous(), grad_output = grad_output_.contiguous();
     Tensor grad_sites = at::zeros({sites.size(0), 10}, sites.options());
+    if (records_pay(width * height, sites.size(0))) {
+        Tensor scratch = scratch_for(sites, sad_site_scratch_bytes(u32(sites.size(0))));
+        ok(sad_render_backward_in(ptr<uint32_t>(cand0), ptr<uint32_t>(cand1), ptr(grad_output), ptr(grad_sites),
+                                  ptr(sites), static_cast<float>(inv_scale_sq), u32(sites.size(0)),
+                                  static_cast<int>(width), static_cast<int>(height), static_cast<int>(width),
+                                  static_cast<int>(height), scratch.data_ptr(), static_cast<size_t>(scratch.numel()),
+                                  stream_of(cand0)));
+        return grad_sites;
+    }
     ok(sad_render_backward(ptr<uint32_t>(cand0), ptr<uint32_t>(cand1), ptr(grad_output), ptr(grad_sites), ptr(sites),
                            static_cast<float>(inv_scale_sq), u32(sites.size(0)), static_cast<int>(width),
                            static_cast<int>(height), static_cast<int>(width), static_cast<int>(height),
@@ -217,7 +239,8 @@ Tensor update_candidates_compact(const Tensor& cand0_in_, const Tensor& cand1_in
         hpp = ptr<uint32_t>(hp);
     }
     // decoding each site once costs a launch: on fields it does not pay for, the pass decodes
-    if (cand_width * cand_height >= kRecordTexels && site_count <= cand_width * cand_height) {
+    if (cand_width * cand_height >= kRecordTexels && site_count <= cand_width * cand_height &&
+        site_count <= packed_sites.size(0)) {
         Tensor scratch = scratch_for(packed_sites, sad_update_candidates_scratch_bytes(u32(site_count)));
         ok(sad_update_candidates_in(
             ptr<uint32_t>(cand0_in), ptr<uint32_t>(cand1_in), ptr<uint32_t>(cand0_out), ptr<uint32_t>(cand1_out),
@@ -324,6 +347,18 @@ Tensor compute_gradients_tiled(const Tensor& cand0_, const Tensor& cand1_, const
     Tensor cand0 = cand0_.contiguous(), cand1 = cand1_.contiguous(), target = target_.contiguous();
     Tensor rendered = rendered_.contiguous(), mask = mask_.contiguous(), sites = sites_.contiguous();
     if (site_count <= 0) site_count = sites.size(0);
+    if (site_count <= sites.size(0) && records_pay(target.size(0) * target.size(1), site_count)) {
+        Tensor scratch = scratch_for(sites, sad_site_scratch_bytes(u32(site_count)));
+        ok(sad_compute_gradients_tiled_in(
+            ptr<uint32_t>(cand0), ptr<uint32_t>(cand1), ptr(target), ptr(rendered), ptr(mask), ptr(grad_pos_x),
+            ptr(grad_pos_y), ptr(grad_log_tau), ptr(grad_radius), ptr(grad_color_r), ptr(grad_color_g),
+            ptr(grad_color_b), ptr(grad_dir_x), ptr(grad_dir_y), ptr(grad_log_aniso), ptr(sites),
+            static_cast<float>(inv_scale_sq), u32(site_count), ptr(removal_delta), u32(compute_removal),
+            static_cast<float>(ssim_weight), static_cast<int>(target.size(1)), static_cast<int>(target.size(0)),
+            static_cast<int>(cand_width), static_cast<int>(cand_height), scratch.data_ptr(),
+            static_cast<size_t>(scratch.numel()), stream_of(cand0)));
+        return grad_pos_x;
+    }
     ok(sad_compute_gradients_tiled(
         ptr<uint32_t>(cand0), ptr<uint32_t>(cand1), ptr(target), ptr(rendered), ptr(mask), ptr(grad_pos_x),
         ptr(grad_pos_y), ptr(grad_log_tau), ptr(grad_radius), ptr(grad_color_r), ptr(grad_color_g),

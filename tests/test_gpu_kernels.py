@@ -275,6 +275,45 @@ def test_vpt_pass_op(ops, orc):
     assert_lists_match(got, want, lambda ids, xs, ys: packed_dist_np(sites, ids, xs, ys, inv), w, h)
 
 
+@pytest.mark.parametrize("w,h,n", [(1024, 512, 9000), (731, 719, 40000)])
+def test_operators_with_site_records(ops, w, h, n):
+    """From 131,072 texels (candidate pass) and 524,288 pixels (render, adjoint, gradients) the
+    operators build site records first: the same lists and image as the calls without, bit for
+    bit, and the same float sums up to their order (FP32: each within some 1e-6 of its norm)."""
+    from sad_gb300 import _lib
+    img, sites = cases.scene(w, h, n, 3)
+    sites[::13, 0] = -1.0
+    inv = 1.0 / max(w, h) ** 2
+    s, c = tf(sites), [t32(x) for x in cases.knn_field(sites, w, h)]
+    vp = lambda t: None if t is None else C.c_void_p(t.data_ptr())
+    packed = torch.empty(n, 8, dtype=torch.float16, device="cuda")
+    ops.pack_candidate_sites(s, packed, n)
+    got, want = [torch.empty_like(x) for x in c], [torch.empty_like(x) for x in c]
+    none = torch.empty(0, dtype=torch.int32, device="cuda")
+    ops.update_candidates_compact(*c, *got, packed, none, none, inv, n, 3 << 16, 0, 1.0, 0, 4, 0, 0, 1, w, h, w, h)
+    _lib.call("sad_update_candidates", *[vp(x) for x in c], *[vp(x) for x in want], vp(packed), n, 3 << 16, inv, 0,
+              1.0, 0, 4, None, None, 0, 0, 1, w, h, w, h, None)
+    torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    image = ops.render_sad(*c, s, inv, w, h)
+    plain = torch.empty_like(image)
+    _lib.call("sad_render", vp(c[0]), vp(c[1]), vp(plain), vp(s), inv, n, w, h, w, h, None)
+    torch.cuda.synchronize()
+    assert torch.equal(image, plain)
+    gout = tf(np.random.default_rng(1).normal(size=(h, w, 3)).astype(np.float32))
+    grad, raw = ops.render_sad_backward(*c, s, gout, inv, w, h), torch.zeros_like(s)
+    _lib.call("sad_render_backward", vp(c[0]), vp(c[1]), vp(gout), vp(raw), vp(s), inv, n, w, h, w, h, None)
+    mask, target = torch.ones(h, w, device="cuda"), tf(img)
+    bufs, plain_bufs = _grad_buffers(n), _grad_buffers(n)
+    ops.compute_gradients_tiled(*c, target, image, mask, s, *bufs, inv, n, 0, 0.0, w, h)
+    _lib.call("sad_compute_gradients_tiled", vp(c[0]), vp(c[1]), vp(target), vp(image), vp(mask),
+              *[vp(b) for b in plain_bufs[:10]], vp(s), inv, n, vp(plain_bufs[10]), 0, 0.0, w, h, w, h, None)
+    torch.cuda.synchronize()
+    for a, b in list(zip(grad.T, raw.T)) + list(zip(bufs[:10], plain_bufs[:10])):
+        assert (a - b).double().norm() <= 1e-5 * b.double().norm()
+
+
 # ---------------------------------------------------------------------------
 # training kernels
 # ---------------------------------------------------------------------------
