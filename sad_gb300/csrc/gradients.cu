@@ -227,7 +227,8 @@ __device__ __forceinline__ void candidate_values(const SiteGeom& g, float3 col, 
 // with SSIM and removal deltas 332 instead of 555 us.  Four blocks per SM (64 registers):
 // three take 197 and 338 us.
 template <class Src, bool kRemoval, bool kSSIM>
-__global__ void __launch_bounds__(256, 4) fused_gradients_kernel(GradParams prm, Src src) {
+__global__ void __launch_bounds__(256, 4)
+    fused_gradients_kernel(const __grid_constant__ GradParams prm, Src src) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int2 at = sum_patch_pixel(lane);
     const int x = blockIdx.x * 32 + (warp & 3) * 8 + at.x;
@@ -267,15 +268,17 @@ __global__ void __launch_bounds__(256, 4) fused_gradients_kernel(GradParams prm,
         for (int i = 0; i < kCand; ++i)
             if (!(valid >> i & 1u) || (wts[i] == 0.0f && rem[i] == 0.0f && (finite >> i & 1u))) ids[i] = kEmpty;
     }
+    const auto load = [=](uint32_t id, SiteGeom& g, float3& c) {
+        src.load(id, g, c);
+        if (!(g.l1 >= 1e-8f)) g.l2 = 1.0f / 1e-8f;  // l2 = 1 / max(l1, 1e-8) (gradients.cu:383)
+    };
     add_site_gradients<kRemoval>(
-        ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred,
-        [&](uint32_t id, SiteGeom& g, float3& c) {
-            src.load(id, g, c);
-            if (!(g.l1 >= 1e-8f)) g.l2 = 1.0f / 1e-8f;  // l2 = 1 / max(l1, 1e-8) (gradients.cu:383)
-        },
-        [&](uint32_t id, int k, float v) {
-            float* to = k < 10 ? prm.soa[k < 10 ? k : 0] : prm.removal;
-            atomicAdd(to + id, v);
+        ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred, load,
+        [&](uint32_t id, int k, float v) { atomicAdd((k < 10 ? prm.soa[k < 10 ? k : 0] : prm.removal) + id, v); },
+        [&](const LeftCandidates& left) {
+            add_by_table<kRemoval>(left, load, [p = &prm](uint32_t id, int k, float v) {
+                atomicAdd((k < 10 ? p->soa[k < 10 ? k : 0] : p->removal) + id, v);
+            });
         });
 }
 

@@ -197,9 +197,9 @@ void launch_clear_candidates(uint32_t* c0, uint32_t* c1, int w, int h, cudaStrea
 // autograd adjoint (backends/pytorch/torch_ext/cuda/sad_bindings.cu:41-207)
 // ---------------------------------------------------------------------------
 // Each warp takes an 8x4 patch and sums its sites' gradients by itself (warp_sums.cuh).  Bound
-// by issue (79% at 1999x1503): 327 us there with 46,941 sites and 44 us at 512x512 with 16,384,
-// against 875 and 93 us with a key table and float adds in shared memory.  Four blocks per SM
-// (64 registers): three and five are 6% and 2% slower.
+// by issue (79% at 1999x1503): 327 us there with 46,941 raw sites (290 us from site records) and
+// 44 us at 512x512 with 16,384, against 875 and 93 us with a key table and float adds in shared
+// memory.  Four blocks per SM (64 registers): three and five are 6% and 2% slower.
 template <class Src>
 __global__ void __launch_bounds__(256, 4) render_backward_kernel(
     const uint4* __restrict__ cand0, const uint4* __restrict__ cand1,
@@ -273,10 +273,12 @@ __global__ void __launch_bounds__(256, 4) render_backward_kernel(
             if (!(valid >> i & 1u) || (wts[i] == 0.0f && logits[i] > -INFINITY)) ids[i] = kEmpty;
     }
     float rem[kCand];
-    add_site_gradients<false>(
-        ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred,
-        [&](uint32_t id, SiteGeom& g, float3& c) { src.load(id, g, c); },
-        [&](uint32_t id, int k, float v) { atomicAdd(grad_sites + static_cast<size_t>(id) * 10 + k, v); });
+    const auto load = [=](uint32_t id, SiteGeom& g, float3& c) { src.load(id, g, c); };
+    const auto add = [=](uint32_t id, int k, float v) {
+        atomicAdd(grad_sites + static_cast<size_t>(id) * 10 + k, v);
+    };
+    add_site_gradients<false>(ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred, load, add,
+                              [&](const LeftCandidates& left) { add_by_table<false>(left, load, add); });
 }
 
 template <class Src>

@@ -10,9 +10,12 @@
 // What is the same for every pixel of a site (softness, scales) is multiplied in after the
 // sum.  Groups of 8 balance the site loop's length, which falls with the group (fewer
 // distinct sites, fewer idle lanes), against the global reductions, which rise: a 1999x1503
-// render and its adjoint take 431 us, with groups of 4, 16 and 32 lanes 450, 448 and 471 us.
+// render and its adjoint took 431 us, with groups of 4, 16 and 32 lanes 450, 448 and 471 us
+// (from raw sites and without the table).
 // Lists without common sites (a random initial field) would make that loop long: once the
-// first sites turn out to be shared by few lanes, the rest is added lane by lane.
+// first sites turn out to be shared by few lanes, the block collects what is left in a key
+// table in shared memory, whose float adds rarely meet then (added straight to global memory,
+// the terms' arbitrary order would show in more of the sums' last bits).
 #pragma once
 
 #include "accum.cuh"
@@ -22,6 +25,7 @@
 namespace sad {
 
 constexpr int kSumGroup = 8;
+constexpr int kSumSlots = 256;  // keys of the block's table
 
 // Pixel of a lane in its warp's 8x4 patch, with every eight lanes a 4x2 patch.
 __device__ __forceinline__ int2 sum_patch_pixel(int lane) {
@@ -114,13 +118,82 @@ __device__ __forceinline__ uint32_t min8(const uint32_t (&a)[8]) {
     return min(min(min(a[0], a[1]), min(a[2], a[3])), min(min(a[4], a[5]), min(a[6], a[7])));
 }
 
-// Adds the gradients of a warp's pixels (all 32 lanes call it; ids: kEmpty where a slot
-// carries none).  load(id, geom, colour) reads a site; add(id, k, value) adds to value k of a
-// site: its ten parameters and, with kRemoval, rem[] as value 10.
+// What the site loop leaves of a pixel's candidates, for add_by_table.
+struct LeftCandidates {
+    uint32_t ids[kCand];
+    float wts[kCand], rem[kCand];
+    float ux, uy, inv_s2, inv_scale;
+    float3 dLdp, pred;
+};
+
+// Adds them through a key table of the block (all 256 threads call it).  A call of its own, and
+// with arguments of its own: inlined, its registers cost the site loop 6% (1999x1503: 419
+// instead of 395 us).
 template <bool kRemoval, class Load, class Add>
+__device__ __noinline__ void add_by_table(const LeftCandidates& left, Load load, Add add) {
+    constexpr int NV = kRemoval ? 11 : 10;
+    uint32_t ids[kCand];
+    float wts[kCand], rem[kCand];
+#pragma unroll
+    for (int i = 0; i < kCand; ++i) {
+        ids[i] = left.ids[i];
+        wts[i] = left.wts[i];
+        if constexpr (kRemoval) rem[i] = left.rem[i];
+    }
+    __shared__ TileTable<NV, kSumSlots, AccFloat> table;
+    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+    table.init(tid, 256);
+    __syncthreads();
+    int slots[kCand];
+#pragma unroll
+    for (int i = 0; i < kCand; ++i) slots[i] = register_key(table, ids[i]);
+    const uint32_t turn = lane_rotation();  // lanes with like lists visit different sites at a step
+    rotate8(ids, turn);
+    rotate8(wts, turn);
+    rotate8(slots, turn);
+    if constexpr (kRemoval) rotate8(rem, turn);
+#pragma unroll 1
+    for (int j = 0; j < kCand; ++j) {
+        if (ids[0] != kEmpty) {
+            SiteGeom g;
+            float3 col;
+            load(ids[0], g, col);
+            float o[10], v[NV];
+            candidate_grads(g, col, left.ux, left.uy, left.inv_s2, left.inv_scale, wts[0], left.dLdp, left.pred, false,
+                            o);
+#pragma unroll
+            for (int k = 0; k < 10; ++k) v[k] = o[k];
+            if constexpr (kRemoval) v[10] = rem[0];
+            if (slots[0] >= 0) {
+                table.add(slots[0], v);
+            } else {
+#pragma unroll
+                for (int k = 0; k < NV; ++k) add(ids[0], k, v[k]);
+            }
+        }
+        shift8(ids);
+        shift8(wts);
+        shift8(slots);
+        if constexpr (kRemoval) shift8(rem);
+    }
+    __syncthreads();
+    const int used = table.size();
+    for (int q = tid; q < used * NV; q += 256) {
+        const int d = q / NV, k = q - d * NV;
+        add(table.key_at(d), k, table.value(k, d));
+    }
+}
+
+
+// Adds the gradients of a block's pixels (all 256 threads call it; ids: kEmpty where a slot
+// carries none).  load(id, geom, colour) reads a site; add(id, k, value) adds to value k of a
+// site: its ten parameters and, with kRemoval, rem[] as value 10; by_table(left) calls
+// add_by_table.
+template <bool kRemoval, class Load, class Add, class Table>
 __device__ __forceinline__ void add_site_gradients(uint32_t (&ids)[kCand], float (&wts)[kCand],
                                                    float (&rem)[kCand], float ux, float uy, float inv_s2,
-                                                   float inv_scale, float3 dLdp, float3 pred, Load load, Add add) {
+                                                   float inv_scale, float3 dLdp, float3 pred, Load load, Add add,
+                                                   Table by_table) {
     constexpr int NV = kRemoval ? 11 : 10, G = kSumGroup, R = FoldedCount<NV, G>::value;
     constexpr uint32_t full = 0xffffffffu;
     const uint32_t lane = lane_id();
@@ -130,13 +203,17 @@ __device__ __forceinline__ void add_site_gradients(uint32_t (&ids)[kCand], float
     bool by_tau[R];
 #pragma unroll
     for (int k = 0; k < R; ++k) scale[k] = sum_scale(first + k, inv_s2, inv_scale, by_tau[k]);
+    // over the first two rounds, at least half a lane's pixel of those that list anything
+    const int enough = __popc(__ballot_sync(full, min8(ids) != kEmpty)) / 2;
     int rounds = 0, members = 0;
+    bool left = true;
 #pragma unroll 1
-    while (rounds < 8 || members >= 64) {  // 64: on average two lanes of a group
+    while (rounds < 2 || members >= enough) {
         uint32_t id = min8(ids);
 #pragma unroll
         for (int m = G / 2; m > 0; m /= 2) id = min(id, __shfl_xor_sync(full, id, m));
-        if (!__any_sync(full, id != kEmpty)) return;
+        left = __any_sync(full, id != kEmpty) != 0;
+        if (!left) break;
         float w = 0.0f, r = 0.0f;
         bool mine = false;
 #pragma unroll
@@ -149,7 +226,7 @@ __device__ __forceinline__ void add_site_gradients(uint32_t (&ids)[kCand], float
             }
         }
         mine &= id != kEmpty;
-        if (rounds < 8) {
+        if (rounds < 2) {
             members += __popc(__ballot_sync(full, mine));
             ++rounds;
         }
@@ -173,23 +250,21 @@ __device__ __forceinline__ void add_site_gradients(uint32_t (&ids)[kCand], float
         for (int k = 0; k < R; ++k)
             if (k < count && id != kEmpty) add(id, first + k, s[k] * (scale[k] * (by_tau[k] ? tau : 1.0f)));
     }
-#pragma unroll 1
-    for (int slot = 0; slot < kCand; ++slot) {
-        if (ids[0] != kEmpty) {
-            SiteGeom g;
-            float3 col;
-            load(ids[0], g, col);
-            float v[10];
-            candidate_grads(g, col, ux, uy, inv_s2, inv_scale, wts[0], dLdp, pred, false, v);
+    if (!__syncthreads_or(left)) return;
+    LeftCandidates rest;
 #pragma unroll
-            for (int k = 0; k < 10; ++k) add(ids[0], k, v[k]);
-            if constexpr (kRemoval) add(ids[0], 10, rem[0]);
-        }
-        shift8(ids);
-        shift8(wts);
-        if constexpr (kRemoval) shift8(rem);
-        ids[kCand - 1] = kEmpty;
+    for (int i = 0; i < kCand; ++i) {
+        rest.ids[i] = ids[i];
+        rest.wts[i] = wts[i];
+        if constexpr (kRemoval) rest.rem[i] = rem[i];
     }
+    rest.ux = ux;
+    rest.uy = uy;
+    rest.inv_s2 = inv_s2;
+    rest.inv_scale = inv_scale;
+    rest.dLdp = dLdp;
+    rest.pred = pred;
+    by_table(rest);
 }
 
 }  // namespace sad

@@ -280,6 +280,7 @@ def test_operators_with_site_records(ops, w, h, n):
     """From 131,072 texels (candidate pass) and 524,288 pixels (render, adjoint, gradients) the
     operators build site records first: the same lists and image as the calls without, bit for
     bit, and the same float sums up to their order (FP32: each within some 1e-6 of its norm)."""
+    import ctypes as C
     from sad_gb300 import _lib
     img, sites = cases.scene(w, h, n, 3)
     sites[::13, 0] = -1.0
