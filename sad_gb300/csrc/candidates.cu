@@ -347,7 +347,13 @@ __device__ __forceinline__ void vpt_pixel(const VptParams& prm, const Src& src, 
         bi[0] = a.x; bi[1] = a.y; bi[2] = a.z; bi[3] = a.w;
         bi[4] = b.x; bi[5] = b.y; bi[6] = b.z; bi[7] = b.w;
     }
-    sorted_own_list<8>(bi, bd, n, [&](uint32_t id) { return vpt_distance(src, id, ux, uy, inv_s2, inv_scale); });
+    if (prm.have_distances) {
+        const float4 a = prm.distances[2 * p], b = prm.distances[2 * p + 1];
+        bd[0] = a.x; bd[1] = a.y; bd[2] = a.z; bd[3] = a.w;
+        bd[4] = b.x; bd[5] = b.y; bd[6] = b.z; bd[7] = b.w;
+    } else {
+        sorted_own_list<8>(bi, bd, n, [&](uint32_t id) { return vpt_distance(src, id, ux, uy, inv_s2, inv_scale); });
+    }
 
     const int j = static_cast<int>(jump);
 #pragma unroll 1
@@ -420,6 +426,10 @@ __device__ __forceinline__ void vpt_pixel(const VptParams& prm, const Src& src, 
     }
     reinterpret_cast<uint4*>(prm.out0)[p] = make_uint4(bi[0], bi[1], bi[2], bi[3]);
     reinterpret_cast<uint4*>(prm.out1)[p] = make_uint4(bi[4], bi[5], bi[6], bi[7]);
+    if (prm.distances) {
+        prm.distances[2 * p] = make_float4(bd[0], bd[1], bd[2], bd[3]);
+        prm.distances[2 * p + 1] = make_float4(bd[4], bd[5], bd[6], bd[7]);
+    }
 }
 
 // Pixel of a thread in a 32x8-pixel block of eight warps: each warp takes an 8x4 patch, whose

@@ -22,6 +22,7 @@ struct RenderScratch {
     SiteGeom* vgeom;
     uint32_t* c0[2];
     uint32_t* c1[2];
+    float4* distances;  // of the last pass's candidates
     uint32_t* horder;
     uint32_t* hpos;
     uint32_t* hpairs;
@@ -47,6 +48,7 @@ static RenderScratch carve(void* base, uint32_t n, int cw, int ch) {
         r.c0[b] = reinterpret_cast<uint32_t*>(take(nc));
         r.c1[b] = reinterpret_cast<uint32_t*>(take(nc));
     }
+    r.distances = reinterpret_cast<float4*>(take(2 * nc));
     r.horder = reinterpret_cast<uint32_t*>(take(static_cast<size_t>(n) * 4));
     r.hpos = reinterpret_cast<uint32_t*>(take(static_cast<size_t>(n) * 4));
     r.hpairs = reinterpret_cast<uint32_t*>(take(static_cast<size_t>(padded) * 8));
@@ -145,7 +147,9 @@ static sad_status_t render_from_sites_impl(const sad_render_config_t* cfg, const
         p.width = cw;
         p.height = ch;
         p.state = nullptr;
+        p.distances = r.distances;
         for (int i = 0; i < this_passes; ++i) {
+            p.have_distances = i > 0;  // a round's first pass reads the flood's field
             p.step = sad_pack_jump_step(jump_pass, cw, ch);
             p.step_high = jump_pass >> 16;
             p.in0 = r.c0[a];
