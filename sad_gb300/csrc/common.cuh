@@ -94,6 +94,7 @@ __host__ __device__ __forceinline__ uint32_t xorshift32(uint32_t x) {
 
 // Candidate-field texel of an output pixel, backends/cuda/src/sad_common.cuh:113-125.
 __device__ __forceinline__ int cand_index_for_pixel(int x, int y, int w, int h, int cw, int ch) {
+    if (cw == w && ch == h) return y * w + x;  // the usual field, without two integer divisions
     int sw = w > 0 ? w : 1;
     int sh = h > 0 ? h : 1;
     int cx = clampi((x * cw) / sw, 0, cw - 1);
