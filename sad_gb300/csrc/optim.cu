@@ -366,51 +366,101 @@ void launch_adam_soa(Site* sites, float* adam, const float* const g[10], const A
 // which are consumed and cleared (slots 0-9; slots 10-11, the removal delta, belong to the
 // prune step), then the refreshed SiteGeom / SiteColor records.  Inactive sites carry no
 // gradient and are left untouched.
-__device__ __forceinline__ void adam_train_one(Site* __restrict__ sites, float* __restrict__ adam,
-                                               long long* __restrict__ fix12, const TauLists& tl,
-                                               const float* __restrict__ tau_gin, SiteGeom* __restrict__ geom,
-                                               SiteColor* __restrict__ color, const AdamHyper& hp,
-                                               const DevState* __restrict__ state, int iterations, int w, int h,
-                                               uint32_t i);
+//
+// A warp takes 32 sites of the active list.  Their rows (80 bytes of Adam state, 80 of a
+// gradient record, 40 of the site) come and go through shared memory in chunks of a fifth of
+// a row, neighbouring lanes neighbouring chunks, so that an instruction touches a few lines
+// instead of one per lane; the copies in run while the tau pass gathers.  Bound by latency and
+// the gathers.  (One row per lane kept the load queue full at 9% issue and 30% of L2's rate.)
+constexpr int kAdamThreads = 128;
 
-__global__ void adam_train_kernel(Site* __restrict__ sites, float* __restrict__ adam,
-                                  long long* __restrict__ fix12, TauLists tl,
-                                  const float* __restrict__ tau_gin, SiteGeom* __restrict__ geom,
-                                  SiteColor* __restrict__ color, AdamHyper hp,
-                                  const DevState* __restrict__ state, int iterations, int w, int h) {
-    pdl_wait();
-    const uint32_t n_alive = state->n_alive;
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n_alive; j += gridDim.x * blockDim.x)
-        adam_train_one(sites, adam, fix12, tl, tau_gin, geom, color, hp, state, iterations, w, h, tl.alive[j]);
+struct AdamStage {  // of one warp
+    float4 adam[32][5];
+    longlong2 grads[32][5];
+    float2 site[32][5];
+};
+
+__device__ __forceinline__ void copy_async16(void* shared, const void* global) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                     static_cast<uint32_t>(__cvta_generic_to_shared(shared))),
+                 "l"(global)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_async8(void* shared, const void* global) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                     static_cast<uint32_t>(__cvta_generic_to_shared(shared))),
+                 "l"(global)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// All lanes of the warp; i: the lane's site, kEmpty for none.
+__device__ __forceinline__ void adam_train_warp(Site* __restrict__ sites, float* __restrict__ adam,
+                                                long long* __restrict__ fix12, const TauLists& tl,
+                                                const float* __restrict__ tau_gin, SiteGeom* __restrict__ geom,
+                                                SiteColor* __restrict__ color, const AdamHyper& hp,
+                                                const DevState* __restrict__ state, int iterations, int w, int h,
+                                                uint32_t i, AdamStage& stage) {
+    const uint32_t lane = lane_id();
+    float4* const adam_rows = &stage.adam[0][0];
+    longlong2* const grad_rows = &stage.grads[0][0];
+    float2* const site_rows = &stage.site[0][0];
+    __syncwarp();  // the last sites' chunks are out
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+        const uint32_t c = lane + 32 * j, part = c % 5;
+        const uint32_t id = __shfl_sync(0xffffffffu, i, c / 5);
+        if (id == kEmpty) continue;
+        copy_async16(grad_rows + c, reinterpret_cast<const longlong2*>(fix12 + static_cast<size_t>(id) * 12) + part);
+        copy_async16(adam_rows + c, reinterpret_cast<const float4*>(adam + static_cast<size_t>(id) * 20) + part);
+        copy_async8(site_rows + c, reinterpret_cast<const float2*>(sites + id) + part);
+    }
+    float tau_g = 0.0f;
+    if (i != kEmpty) tau_g = tau_list_pass(tl, tau_gin, i, tau_lambda(state->iter, iterations));
+    copy_async_wait();
+    __syncwarp();
+    if (i != kEmpty) {
+        const float norm = 1.0f / static_cast<float>(w * h);
+        longlong2 q[5];
+#pragma unroll
+        for (int k = 0; k < 5; ++k) q[k] = stage.grads[lane][k];
+        float g[10] = {from_fix(q[0].x) * norm, from_fix(q[0].y) * norm, tau_g * norm,
+                       from_fix(q[1].y) * norm, from_fix(q[2].x) * norm, from_fix(q[2].y) * norm,
+                       from_fix(q[3].x) * norm, from_fix(q[3].y) * norm, from_fix(q[4].x) * norm,
+                       from_fix(q[4].y) * norm};
+        Site s = site_load(reinterpret_cast<const Site*>(site_rows), lane);
+        const float c1 = state->adam_c1, c2 = state->adam_c2;
+        AdamSlots a;
+        adam_load(reinterpret_cast<const float*>(adam_rows), lane, a);
+        adam_site(s, a, g, hp, c1, c2, w, h);
+        adam_store(reinterpret_cast<float*>(adam_rows), lane, a);
+        site_store(reinterpret_cast<Site*>(site_rows), lane, s);
+        store_geom(geom, i, make_geom(s.px, s.py, s.log_tau, s.radius, s.dx, s.dy, s.log_aniso));
+        reinterpret_cast<float4*>(color)[i] = make_float4(s.r, s.g, s.b, 0.0f);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+        const uint32_t c = lane + 32 * j, part = c % 5;
+        const uint32_t id = __shfl_sync(0xffffffffu, i, c / 5);
+        if (id == kEmpty) continue;
+        reinterpret_cast<longlong2*>(fix12 + static_cast<size_t>(id) * 12)[part] = make_longlong2(0, 0);
+        reinterpret_cast<float4*>(adam + static_cast<size_t>(id) * 20)[part] = adam_rows[c];
+        reinterpret_cast<float2*>(sites + id)[part] = site_rows[c];
+    }
 }
 
-__device__ __forceinline__ void adam_train_one(Site* __restrict__ sites, float* __restrict__ adam,
-                                               long long* __restrict__ fix12, const TauLists& tl,
-                                               const float* __restrict__ tau_gin, SiteGeom* __restrict__ geom,
-                                               SiteColor* __restrict__ color, const AdamHyper& hp,
-                                               const DevState* __restrict__ state, int iterations, int w, int h,
-                                               uint32_t i) {
-    const float tau_g = tau_list_pass(tl, tau_gin, i, tau_lambda(state->iter, iterations));
-    float norm = 1.0f / static_cast<float>(w * h);
-    longlong2* gq = reinterpret_cast<longlong2*>(fix12 + static_cast<size_t>(i) * 12);
-    longlong2 q[5];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) q[k] = gq[k];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) gq[k] = make_longlong2(0, 0);
-    float g[10] = {from_fix(q[0].x) * norm, from_fix(q[0].y) * norm, tau_g * norm,
-                   from_fix(q[1].y) * norm, from_fix(q[2].x) * norm, from_fix(q[2].y) * norm,
-                   from_fix(q[3].x) * norm, from_fix(q[3].y) * norm, from_fix(q[4].x) * norm,
-                   from_fix(q[4].y) * norm};
-    Site s = site_load(sites, i);
-    const float c1 = state->adam_c1, c2 = state->adam_c2;
-    AdamSlots a;
-    adam_load(adam, i, a);
-    adam_site(s, a, g, hp, c1, c2, w, h);
-    adam_store(adam, i, a);
-    site_store(sites, i, s);
-    store_geom(geom, i, make_geom(s.px, s.py, s.log_tau, s.radius, s.dx, s.dy, s.log_aniso));
-    reinterpret_cast<float4*>(color)[i] = make_float4(s.r, s.g, s.b, 0.0f);
+__global__ void __launch_bounds__(kAdamThreads)
+    adam_train_kernel(Site* __restrict__ sites, float* __restrict__ adam, long long* __restrict__ fix12, TauLists tl,
+                      const float* __restrict__ tau_gin, SiteGeom* __restrict__ geom, SiteColor* __restrict__ color,
+                      AdamHyper hp, const DevState* __restrict__ state, int iterations, int w, int h) {
+    __shared__ AdamStage stage[kAdamThreads / 32];
+    pdl_wait();
+    const uint32_t n_alive = state->n_alive;
+    // whole warps: j differs by the lane only
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; (j & ~31u) < n_alive; j += gridDim.x * blockDim.x)
+        adam_train_warp(sites, adam, fix12, tl, tau_gin, geom, color, hp, state, iterations, w, h,
+                        j < n_alive ? tl.alive[j] : kEmpty, stage[threadIdx.x / 32]);
 }
 
 void launch_adam_train(Site* sites, float* adam, long long* fix12, const uint32_t* nbr,
@@ -420,8 +470,8 @@ void launch_adam_train(Site* sites, float* adam, long long* fix12, const uint32_
                        cudaStream_t st) {
     if (max_alive == 0) return;
     TauLists tl{reinterpret_cast<uint4*>(const_cast<uint32_t*>(nbr)), const_cast<float*>(raw), alive};
-    launch_pdl(adam_train_kernel, dim3(blocks_for(max_alive, 256)), dim3(256), 0, st, sites, adam, fix12, tl,
-               tau_gin, geom, color, hp, state, iterations, w, h);
+    launch_pdl(adam_train_kernel, dim3(blocks_for(max_alive, kAdamThreads)), dim3(kAdamThreads), 0, st, sites, adam,
+               fix12, tl, tau_gin, geom, color, hp, state, iterations, w, h);
     note_launches(1);
 }
 
@@ -540,18 +590,25 @@ __global__ void __launch_bounds__(256) tau_list_batch_kernel(const SiteBatchItem
     }
 }
 
-__global__ void __launch_bounds__(256) adam_batch_kernel(const SiteBatchItem* __restrict__ items,
-                                                         const uint32_t* __restrict__ prefix, uint32_t n_items,
-                                                         AdamHyper hp, int iterations) {
+__global__ void __launch_bounds__(kAdamThreads) adam_batch_kernel(const SiteBatchItem* __restrict__ items,
+                                                                  const uint32_t* __restrict__ prefix,
+                                                                  uint32_t n_items, AdamHyper hp, int iterations) {
     pdl_wait();
     __shared__ uint32_t s_prefix[kMaxBatchItems + 1];
+    __shared__ AdamStage stage[kAdamThreads / 32];
     const uint32_t total = load_site_prefix(s_prefix, prefix, n_items);
-    for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
-        const uint32_t k = batch_item_of(s_prefix, n_items, g);
-        const SiteBatchItem& it = items[k];
-        TauLists tl{reinterpret_cast<uint4*>(it.tau_nbr), it.tau_raw, it.alive};
-        adam_train_one(it.sites, it.adam, it.grads, tl, it.tau_a, it.geom, it.color, hp, it.state, iterations, it.w,
-                       it.h, it.alive[g - s_prefix[k]]);
+    for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; (g & ~31u) < total; g += gridDim.x * blockDim.x) {
+        // one image after the other: a warp's sites are mostly one image's
+        const uint32_t mine = g < total ? batch_item_of(s_prefix, n_items, g) : kEmpty;
+        uint32_t todo = __ballot_sync(0xffffffffu, mine != kEmpty);
+        while (todo != 0u) {
+            const uint32_t k = __shfl_sync(0xffffffffu, mine, __ffs(todo) - 1);
+            const SiteBatchItem& it = items[k];
+            TauLists tl{reinterpret_cast<uint4*>(it.tau_nbr), it.tau_raw, it.alive};
+            adam_train_warp(it.sites, it.adam, it.grads, tl, it.tau_a, it.geom, it.color, hp, it.state, iterations,
+                            it.w, it.h, mine == k ? it.alive[g - s_prefix[k]] : kEmpty, stage[threadIdx.x / 32]);
+            todo &= ~__ballot_sync(0xffffffffu, mine == k);
+        }
     }
 }
 
@@ -584,8 +641,8 @@ void launch_tau_list_batch(const SiteBatchItem* items, const uint32_t* site_pref
 
 void launch_adam_batch(const SiteBatchItem* items, const uint32_t* site_prefix, uint32_t n_items,
                        const AdamHyper& hp, int iterations, uint32_t grid_threads, cudaStream_t st) {
-    launch_pdl(adam_batch_kernel, dim3(batch_grid(grid_threads)), dim3(256), 0, st, items, site_prefix, n_items, hp,
-               iterations);
+    launch_pdl(adam_batch_kernel, dim3(std::max(1u, blocks_for(grid_threads, kAdamThreads))), dim3(kAdamThreads), 0,
+               st, items, site_prefix, n_items, hp, iterations);
     note_launches(1);
 }
 
