@@ -31,6 +31,10 @@ namespace sad {
 constexpr int kFixFracBits = 24;
 constexpr float kFixScale = 16777216.0f;                  // 2^24
 constexpr float kFixInvScale = 5.9604644775390625e-08f;  // 2^-24
+// The log_tau word of an inactive site's record (which no gradient is added to): the tau passes
+// read a neighbour's gradient and whether it is active in one gather.
+constexpr long long kInactiveWord = -0x7fffffffffffffffll - 1;
+constexpr int kTauWord = 2;
 // Per tile, a fixed-point sum is kept as two 32-bit words (hi * 2^20 + lo): shared
 // memory has native 32-bit integer atomics but no native 64-bit add.  Exact while a tile's
 // sum of one value stays below 2^27 in magnitude (and each term below 2^27).

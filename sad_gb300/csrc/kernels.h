@@ -300,9 +300,10 @@ void launch_prune_pairs_alive(long long* fix12, float fix_mul, uint32_t* pairs, 
                               const DevState* state, uint32_t max_alive, float delta_norm, cudaStream_t st);
 // trainer form: prune the first prune_k[state->iter] entries of sorted pairs, also in the
 // prepared and the VPT geometry
-void launch_prune_sorted_train(Site* sites, SiteGeom* geom, SiteGeom* vgeom, const uint32_t* pairs,
-                               const uint32_t* prune_k, const DevState* state, uint32_t max_k,
-                               cudaStream_t st);
+void launch_prune_sorted_train(Site* sites, SiteGeom* geom, SiteGeom* vgeom, long long* fix12,
+                               const uint32_t* pairs, const uint32_t* prune_k, const DevState* state,
+                               uint32_t max_k, cudaStream_t st);
+void launch_mark_inactive(const Site* sites, long long* fix12, uint32_t n, cudaStream_t st);
 // stream compaction of the active set: alive = ascending active slots of [0, n) (prepared
 // geometry px >= 0), *n_alive = their number; block_counts holds compact_blocks(n) words
 uint32_t compact_blocks(uint32_t n);

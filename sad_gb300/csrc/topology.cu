@@ -185,11 +185,11 @@ void launch_prune_by_index(Site* sites, const uint32_t* idx, uint32_t k, cudaStr
 
 // Trainer form: write-indices + prune fused; the count comes from the host-planned
 // per-iteration table (the schedule is fixed before the fit starts).
-// The pruned sites are marked inactive in the site records, the prepared geometry and
-// the VPT geometry (the refresh repacks only listed sites).
+// The pruned sites are marked inactive in the site records, the prepared geometry, the VPT
+// geometry (the refresh repacks only listed sites) and the gradient records.
 __global__ void prune_sorted_kernel(Site* __restrict__ sites, SiteGeom* __restrict__ geom,
-                                    SiteGeom* __restrict__ vgeom, const uint2* __restrict__ pairs,
-                                    const uint32_t* __restrict__ prune_k,
+                                    SiteGeom* __restrict__ vgeom, long long* __restrict__ fix12,
+                                    const uint2* __restrict__ pairs, const uint32_t* __restrict__ prune_k,
                                     const DevState* __restrict__ state) {
     pdl_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -203,6 +203,19 @@ __global__ void prune_sorted_kernel(Site* __restrict__ sites, SiteGeom* __restri
     geom[s].py = -1.0f;
     vgeom[s].px = -1.0f;
     vgeom[s].py = -1.0f;
+    fix12[static_cast<size_t>(s) * 12 + kTauWord] = kInactiveWord;
+}
+
+// Marks the gradient records of the sites that are not active.
+__global__ void mark_inactive_kernel(const Site* __restrict__ sites, long long* __restrict__ fix12, uint32_t n) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n && !(sites[i].px >= 0.0f)) fix12[static_cast<size_t>(i) * 12 + kTauWord] = kInactiveWord;
+}
+
+void launch_mark_inactive(const Site* sites, long long* fix12, uint32_t n, cudaStream_t st) {
+    if (n == 0) return;
+    mark_inactive_kernel<<<blocks_for(n, 256), 256, 0, st>>>(sites, fix12, n);
+    note_launches(1);
 }
 
 // Batched form: blockIdx.y is the image; each marks the first prune_k[iter] of its pairs.
@@ -220,6 +233,7 @@ __global__ void prune_sorted_batch_kernel(const SiteBatchItem* __restrict__ item
     it.geom[s].py = -1.0f;
     it.vgeom[s].px = -1.0f;
     it.vgeom[s].py = -1.0f;
+    it.grads[static_cast<size_t>(s) * 12 + kTauWord] = kInactiveWord;
 }
 
 void launch_prune_sorted_batch(const SiteBatchItem* items, uint32_t n_items, uint32_t max_k, cudaStream_t st) {
@@ -228,12 +242,12 @@ void launch_prune_sorted_batch(const SiteBatchItem* items, uint32_t n_items, uin
     note_launches(1);
 }
 
-void launch_prune_sorted_train(Site* sites, SiteGeom* geom, SiteGeom* vgeom, const uint32_t* pairs,
-                               const uint32_t* prune_k, const DevState* state, uint32_t max_k,
-                               cudaStream_t st) {
+void launch_prune_sorted_train(Site* sites, SiteGeom* geom, SiteGeom* vgeom, long long* fix12,
+                               const uint32_t* pairs, const uint32_t* prune_k, const DevState* state,
+                               uint32_t max_k, cudaStream_t st) {
     if (max_k == 0) return;
     launch_pdl(prune_sorted_kernel, dim3(blocks_for(max_k, 256)), dim3(256), 0, st, sites, geom, vgeom,
-               reinterpret_cast<const uint2*>(pairs), prune_k, state);
+               fix12, reinterpret_cast<const uint2*>(pairs), prune_k, state);
     note_launches(1);
 }
 

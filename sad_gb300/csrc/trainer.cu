@@ -273,7 +273,7 @@ static int iteration_body(sad_trainer* t, bool upd, bool prune, int field, int a
         float delta_norm = 1.0f / std::max(1.0f, t->mask_sum);
         launch_prune_pairs_alive(t->grads, t->removal_mul, t->pairs, t->alive, t->state, hint, delta_norm, s);
         launch_radix_sort_dev(t->pairs, t->n, n_alive_ptr(t), 0xFFFFFFFFu, t->sort_temp, s);
-        launch_prune_sorted_train(t->sites, t->geom, t->vgeom, t->pairs, t->prune_k, t->state,
+        launch_prune_sorted_train(t->sites, t->geom, t->vgeom, t->grads, t->pairs, t->prune_k, t->state,
                                   SAD_MAX_SPLIT_INDICES, s);
         launch_compact(t, s);
     }
@@ -295,6 +295,10 @@ static sad_status_t run_densify(sad_trainer* t, const IterPlan& p, cudaStream_t 
     launch_write_indices(t->pairs, t->idx, p.split_k, s);
     const float* sp[7] = {st[0], st[2], st[3], st[4], st[5], st[6], st[7]};
     launch_split(t->sites, t->adam, t->idx, p.split_k, sp, t->n, t->target, t->w, t->h, s);
+    // the children's records (marked inactive until now) start at zero
+    SAD_TRY(check_cuda(cudaMemsetAsync(t->grads + static_cast<size_t>(t->n) * 12, 0,
+                                       static_cast<size_t>(p.split_k) * 12 * sizeof(long long), s),
+                       "trainer densify: gradient records"));
     t->n += p.split_k;
     t->active += static_cast<int>(p.split_k);
     launch_prepare_sites(t->sites, t->geom, t->color, t->n, s);
@@ -648,6 +652,7 @@ extern "C" sad_status_t sad_trainer_init(sad_trainer_t* t, const float* sites_ho
     SAD_TRY(check_cuda(cudaMemsetAsync(t->adam, 0, static_cast<size_t>(t->cap) * 80, s), "trainer adam clear"));
     SAD_TRY(check_cuda(cudaMemsetAsync(t->grads, 0, static_cast<size_t>(t->cap) * 12 * sizeof(long long), s),
                        "trainer grad clear"));
+    launch_mark_inactive(t->sites, t->grads, t->cap, s);
     SAD_TRY(check_cuda(cudaMemsetAsync(t->stats_fix, 0, static_cast<size_t>(t->cap) * 8 * sizeof(long long), s),
                        "trainer stats clear"));
     launch_reset_state(t->state, t->cfg.beta1, t->cfg.beta2, s);
