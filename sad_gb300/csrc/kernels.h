@@ -219,6 +219,14 @@ void launch_adam_train(Site* sites, float* adam, long long* fix12, const uint32_
                        SiteGeom* geom, SiteColor* color, const AdamHyper& hp,
                        const DevState* state, int iterations, uint32_t max_alive, int w, int h,
                        cudaStream_t st);
+// The tau passes, Adam and (advance) launch_advance_state's step in one launch, for at most
+// kChainSites sites; prepare_site_chain() once before the first.
+constexpr uint32_t kChainSites = 8192;
+cudaError_t prepare_site_chain();
+void launch_site_chain(const uint32_t* c0, const uint32_t* c1, Site* sites, float* adam, long long* fix12,
+                       uint32_t* nbr, float* raw, const uint32_t* alive, float* tau_a, float* tau_b, SiteGeom* geom,
+                       SiteColor* color, const AdamHyper& hp, DevState* state, int iterations, uint32_t n, int cw,
+                       int ch, int ds, int w, int h, bool advance, uint32_t vpt_passes, cudaStream_t st);
 // Batched per-site launches over the compacted active lists of every image of a batch,
 // walked as one flat list: site_prefix[i] = sum of the n_alive of images < i (in device
 // memory, written by launch_batch_site_prefix after each compaction); grid-stride, so the

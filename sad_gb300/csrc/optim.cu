@@ -159,16 +159,16 @@ __device__ __forceinline__ void tau_first_one(const uint4* __restrict__ c0, cons
 }
 
 // One Jacobi pass of an active site from its recorded neighbour list (sum in candidate
-// order, as the first pass and the reference's kernel).
-__device__ __forceinline__ float tau_list_pass(const TauLists& tl, const float* __restrict__ gin,
-                                               uint32_t i, float lambda) {
+// order, as the first pass and the reference's kernel); gin(i): the last pass's value.
+template <class Gin>
+__device__ __forceinline__ float tau_list_pass(const TauLists& tl, Gin gin, uint32_t i, float lambda) {
     const float r = tl.raw[i];
-    if (!(lambda > 0.0f)) return gin[i];
+    if (!(lambda > 0.0f)) return gin(i);
     uint4 a = tl.nbr[2 * i], b = tl.nbr[2 * i + 1];
     uint32_t ids[kCand] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
     float v[kCand];
 #pragma unroll
-    for (int k = 0; k < kCand; ++k) v[k] = ids[k] == kEmpty ? 0.0f : gin[ids[k]];  // gathers overlap
+    for (int k = 0; k < kCand; ++k) v[k] = ids[k] == kEmpty ? 0.0f : gin(ids[k]);  // gathers overlap
     float sum = 0.0f;
     uint32_t cnt = 0;
 #pragma unroll
@@ -188,7 +188,7 @@ __global__ void tau_list_pass_kernel(TauLists tl, const float* __restrict__ gin,
     const float lambda = tau_lambda(state->iter, iterations);
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n_alive; j += gridDim.x * blockDim.x) {
         const uint32_t i = tl.alive[j];
-        gout[i] = tau_list_pass(tl, gin, i, lambda);
+        gout[i] = tau_list_pass(tl, [gin](uint32_t k) { return gin[k]; }, i, lambda);
     }
 }
 
@@ -392,12 +392,21 @@ __device__ __forceinline__ void copy_async8(void* shared, const void* global) {
 }
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// All lanes of the warp; i: the lane's site, kEmpty for none.
+// The iteration's scalars.
+struct StepScalars {
+    float lambda, c1, c2;
+};
+__device__ __forceinline__ StepScalars step_scalars(const DevState* state, int iterations) {
+    return StepScalars{tau_lambda(state->iter, iterations), state->adam_c1, state->adam_c2};
+}
+
+// All lanes of the warp; i: the lane's site, kEmpty for none; tau_gin(i): the third tau pass's
+// value.
+template <class Gin>
 __device__ __forceinline__ void adam_train_warp(Site* __restrict__ sites, float* __restrict__ adam,
-                                                long long* __restrict__ fix12, const TauLists& tl,
-                                                const float* __restrict__ tau_gin, SiteGeom* __restrict__ geom,
-                                                SiteColor* __restrict__ color, const AdamHyper& hp,
-                                                const DevState* __restrict__ state, int iterations, int w, int h,
+                                                long long* __restrict__ fix12, const TauLists& tl, Gin tau_gin,
+                                                SiteGeom* __restrict__ geom, SiteColor* __restrict__ color,
+                                                const AdamHyper& hp, const StepScalars& step, int w, int h,
                                                 uint32_t i, AdamStage& stage) {
     const uint32_t lane = lane_id();
     float4* const adam_rows = &stage.adam[0][0];
@@ -414,7 +423,7 @@ __device__ __forceinline__ void adam_train_warp(Site* __restrict__ sites, float*
         copy_async8(site_rows + c, reinterpret_cast<const float2*>(sites + id) + part);
     }
     float tau_g = 0.0f;
-    if (i != kEmpty) tau_g = tau_list_pass(tl, tau_gin, i, tau_lambda(state->iter, iterations));
+    if (i != kEmpty) tau_g = tau_list_pass(tl, tau_gin, i, step.lambda);
     copy_async_wait();
     __syncwarp();
     if (i != kEmpty) {
@@ -427,10 +436,9 @@ __device__ __forceinline__ void adam_train_warp(Site* __restrict__ sites, float*
                        from_fix(q[3].x) * norm, from_fix(q[3].y) * norm, from_fix(q[4].x) * norm,
                        from_fix(q[4].y) * norm};
         Site s = site_load(reinterpret_cast<const Site*>(site_rows), lane);
-        const float c1 = state->adam_c1, c2 = state->adam_c2;
         AdamSlots a;
         adam_load(reinterpret_cast<const float*>(adam_rows), lane, a);
-        adam_site(s, a, g, hp, c1, c2, w, h);
+        adam_site(s, a, g, hp, step.c1, step.c2, w, h);
         adam_store(reinterpret_cast<float*>(adam_rows), lane, a);
         site_store(reinterpret_cast<Site*>(site_rows), lane, s);
         store_geom(geom, i, make_geom(s.px, s.py, s.log_tau, s.radius, s.dx, s.dy, s.log_aniso));
@@ -455,10 +463,11 @@ __global__ void __launch_bounds__(kAdamThreads)
     __shared__ AdamStage stage[kAdamThreads / 32];
     pdl_wait();
     const uint32_t n_alive = state->n_alive;
+    const StepScalars step = step_scalars(state, iterations);
     // whole warps: j differs by the lane only
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; (j & ~31u) < n_alive; j += gridDim.x * blockDim.x)
-        adam_train_warp(sites, adam, fix12, tl, tau_gin, geom, color, hp, state, iterations, w, h,
-                        j < n_alive ? tl.alive[j] : kEmpty, stage[threadIdx.x / 32]);
+        adam_train_warp(sites, adam, fix12, tl, [tau_gin](uint32_t k) { return tau_gin[k]; }, geom, color, hp, step,
+                        w, h, j < n_alive ? tl.alive[j] : kEmpty, stage[threadIdx.x / 32]);
 }
 
 void launch_adam_train(Site* sites, float* adam, long long* fix12, const uint32_t* nbr,
@@ -528,6 +537,84 @@ void launch_set_wide_far_refs(DevState* state, int value, cudaStream_t st) {
     note_launches(1);
 }
 
+// The per-site work of an iteration in one launch, for fits of at most kChainSites sites: the
+// three tau passes and Adam, a cluster barrier between them instead of a launch, and the state
+// advance.  One cluster of kChainBlocks blocks (a barrier of which costs far less than a launch
+// boundary); the passes exchange their values through L2.
+constexpr int kChainBlocks = 16;
+constexpr int kChainThreads = 256;
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(kChainThreads)
+    site_chain_kernel(const uint4* __restrict__ c0, const uint4* __restrict__ c1, Site* sites, float* adam,
+                      long long* fix12, TauLists tl, float* tau_a, float* tau_b, SiteGeom* geom, SiteColor* color,
+                      AdamHyper hp, DevState* state, int iterations, uint32_t n, int cw, int ch, int ds, int w, int h,
+                      bool advance, uint32_t vpt_passes) {
+    extern __shared__ __align__(16) unsigned char sad_chain_smem[];
+    pdl_wait();
+    const uint32_t n_alive = state->n_alive;
+    const StepScalars step = step_scalars(state, iterations);
+    const uint32_t first = blockIdx.x * kChainThreads + threadIdx.x, stride = kChainBlocks * kChainThreads;
+    for (uint32_t j = first; j < n_alive; j += stride)
+        tau_first_one(c0, c1, geom, fix12, tl, tau_a, n, tl.alive[j], step.lambda, cw, ch, ds);
+    cluster_barrier();
+    if (advance && first == 0) {  // every block has read the state
+        state->iter += 1u;
+        state->vpt_pass += vpt_passes;
+        set_bias_corrections(state, hp.beta1, hp.beta2);
+    }
+    const float* gin = tau_a;
+    float* gout = tau_b;
+    for (int pass = 0; pass < 2; ++pass) {
+        for (uint32_t j = first; j < n_alive; j += stride) {
+            const uint32_t i = tl.alive[j];
+            gout[i] = tau_list_pass(tl, [gin](uint32_t k) { return __ldcg(gin + k); }, i, step.lambda);
+        }
+        cluster_barrier();
+        gin = tau_b;
+        gout = tau_a;
+    }
+    AdamStage& stage = reinterpret_cast<AdamStage*>(sad_chain_smem)[threadIdx.x / 32];
+    for (uint32_t j = first; (j & ~31u) < n_alive; j += stride)
+        adam_train_warp(sites, adam, fix12, tl, [tau_a](uint32_t k) { return __ldcg(tau_a + k); }, geom, color, hp,
+                        step, w, h, j < n_alive ? tl.alive[j] : kEmpty, stage);
+}
+
+cudaError_t prepare_site_chain() {
+    cudaError_t e = cudaFuncSetAttribute(site_chain_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(site_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(kChainThreads / 32 * sizeof(AdamStage)));
+    return e;
+}
+
+void launch_site_chain(const uint32_t* c0, const uint32_t* c1, Site* sites, float* adam, long long* fix12,
+                       uint32_t* nbr, float* raw, const uint32_t* alive, float* tau_a, float* tau_b, SiteGeom* geom,
+                       SiteColor* color, const AdamHyper& hp, DevState* state, int iterations, uint32_t n, int cw,
+                       int ch, int ds, int w, int h, bool advance, uint32_t vpt_passes, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kChainBlocks);
+    cfg.blockDim = dim3(kChainThreads);
+    cfg.dynamicSmemBytes = kChainThreads / 32 * sizeof(AdamStage);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = kChainBlocks;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    TauLists tl{reinterpret_cast<uint4*>(nbr), raw, alive};
+    cudaLaunchKernelEx(&cfg, site_chain_kernel, reinterpret_cast<const uint4*>(c0), reinterpret_cast<const uint4*>(c1),
+                       sites, adam, fix12, tl, tau_a, tau_b, geom, color, hp, state, iterations, n, cw, ch, ds, w, h,
+                       advance, vpt_passes);
+    note_launches(1);
+}
+
 void launch_advance_state(DevState* state, uint32_t vpt_passes, float beta1, float beta2,
                           cudaStream_t st) {
     launch_pdl(advance_state_kernel, dim3(1), dim3(1), 0, st, state, vpt_passes, beta1, beta2);
@@ -584,7 +671,7 @@ __global__ void __launch_bounds__(256) tau_list_batch_kernel(const SiteBatchItem
         const uint32_t i = it.alive[g - s_prefix[k]];
         const float* gin = a_to_b ? it.tau_a : it.tau_b;
         float* gout = a_to_b ? it.tau_b : it.tau_a;
-        gout[i] = tau_list_pass(tl, gin, i, tau_lambda(it.state->iter, iterations));
+        gout[i] = tau_list_pass(tl, [gin](uint32_t k) { return gin[k]; }, i, tau_lambda(it.state->iter, iterations));
     }
 }
 
@@ -603,8 +690,10 @@ __global__ void __launch_bounds__(kAdamThreads) adam_batch_kernel(const SiteBatc
             const uint32_t k = __shfl_sync(0xffffffffu, mine, __ffs(todo) - 1);
             const SiteBatchItem& it = items[k];
             TauLists tl{reinterpret_cast<uint4*>(it.tau_nbr), it.tau_raw, it.alive};
-            adam_train_warp(it.sites, it.adam, it.grads, tl, it.tau_a, it.geom, it.color, hp, it.state, iterations,
-                            it.w, it.h, mine == k ? it.alive[g - s_prefix[k]] : kEmpty, stage[threadIdx.x / 32]);
+            const float* gin = it.tau_a;
+            adam_train_warp(it.sites, it.adam, it.grads, tl, [gin](uint32_t m) { return gin[m]; }, it.geom, it.color,
+                            hp, step_scalars(it.state, iterations), it.w, it.h,
+                            mine == k ? it.alive[g - s_prefix[k]] : kEmpty, stage[threadIdx.x / 32]);
             todo &= ~__ballot_sync(0xffffffffu, mine == k);
         }
     }

@@ -250,21 +250,29 @@ static int iteration_body(sad_trainer* t, bool upd, bool prune, int field, int a
     if (upd) cudaStreamWaitEvent(s, t->ev_join, 0);
     // 4 Jacobi passes: grads slot 2 -> A -> B -> A -> (inside Adam), over the active list
     const uint32_t hint = t->alive_hint;
+    const AdamHyper hp{t->cfg.lr_pos * t->cfg.lr_scale, t->cfg.lr_tau * t->cfg.lr_scale,
+                       t->cfg.lr_radius * t->cfg.lr_scale, t->cfg.lr_color * t->cfg.lr_scale,
+                       t->cfg.lr_dir * t->cfg.lr_scale, t->cfg.lr_aniso * t->cfg.lr_scale,
+                       t->cfg.beta1, t->cfg.beta2, t->cfg.eps};
+    const bool chain = t->n <= kChainSites;
     {
         NvtxRange r_site("tau diffusion and Adam");
-        launch_tau_first_pass(t->cand0[next], t->cand1[next], t->geom, t->grads, t->tau_nbr, t->tau_raw,
-                              t->alive, t->tau_a, t->n, hint, t->state, t->cfg.iterations, t->cw, t->ch,
-                              t->ds, s);
-        launch_tau_list_pass(t->tau_nbr, t->tau_raw, t->alive, t->tau_a, t->tau_b, hint, t->state,
-                             t->cfg.iterations, s);
-        launch_tau_list_pass(t->tau_nbr, t->tau_raw, t->alive, t->tau_b, t->tau_a, hint, t->state,
-                             t->cfg.iterations, s);
-        AdamHyper hp{t->cfg.lr_pos * t->cfg.lr_scale, t->cfg.lr_tau * t->cfg.lr_scale,
-                     t->cfg.lr_radius * t->cfg.lr_scale, t->cfg.lr_color * t->cfg.lr_scale,
-                     t->cfg.lr_dir * t->cfg.lr_scale, t->cfg.lr_aniso * t->cfg.lr_scale,
-                     t->cfg.beta1, t->cfg.beta2, t->cfg.eps};
-        launch_adam_train(t->sites, t->adam, t->grads, t->tau_nbr, t->tau_raw, t->alive, t->tau_a,
-                          t->geom, t->color, hp, t->state, t->cfg.iterations, hint, t->w, t->h, s);
+        if (chain) {
+            launch_site_chain(t->cand0[next], t->cand1[next], t->sites, t->adam, t->grads, t->tau_nbr, t->tau_raw,
+                              t->alive, t->tau_a, t->tau_b, t->geom, t->color, hp, t->state, t->cfg.iterations, t->n,
+                              t->cw, t->ch, t->ds, t->w, t->h, !prune, static_cast<uint32_t>(adv_passes), s);
+            if (!prune) return next;  // the state is advanced too
+        } else {
+            launch_tau_first_pass(t->cand0[next], t->cand1[next], t->geom, t->grads, t->tau_nbr, t->tau_raw,
+                                  t->alive, t->tau_a, t->n, hint, t->state, t->cfg.iterations, t->cw, t->ch,
+                                  t->ds, s);
+            launch_tau_list_pass(t->tau_nbr, t->tau_raw, t->alive, t->tau_a, t->tau_b, hint, t->state,
+                                 t->cfg.iterations, s);
+            launch_tau_list_pass(t->tau_nbr, t->tau_raw, t->alive, t->tau_b, t->tau_a, hint, t->state,
+                                 t->cfg.iterations, s);
+            launch_adam_train(t->sites, t->adam, t->grads, t->tau_nbr, t->tau_raw, t->alive, t->tau_a,
+                              t->geom, t->color, hp, t->state, t->cfg.iterations, hint, t->w, t->h, s);
+        }
     }
     if (prune) {
         // score, sort and prune the active list (the same sorted prefix as over every slot:
@@ -476,6 +484,7 @@ static size_t carve_trainer(sad_trainer* t, void* base) {
 // Streams, events and kernel attributes once the buffers are in place.
 static sad_status_t finish_create(sad_trainer* t) {
     sad_status_t s = check_cuda(prepare_gradient_kernels(), "trainer kernel attributes");
+    if (s == SAD_OK) s = check_cuda(prepare_site_chain(), "trainer kernel attributes");
     if (s == SAD_OK)
         s = check_cuda(cudaStreamCreateWithFlags(&t->st, cudaStreamNonBlocking), "trainer stream");
     if (s == SAD_OK)
