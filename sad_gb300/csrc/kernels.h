@@ -220,8 +220,11 @@ void launch_adam_train(Site* sites, float* adam, long long* fix12, const uint32_
                        const DevState* state, int iterations, uint32_t max_alive, int w, int h,
                        cudaStream_t st);
 // The tau passes, Adam and (advance) launch_advance_state's step in one launch, for at most
-// kChainSites sites; prepare_site_chain() once before the first.
-constexpr uint32_t kChainSites = 8192;
+// kChainSites sites (one per thread of its cluster); prepare_site_chain() once before the first.
+// Fits of 200 iterations with and without: 128x128 with 1,024 sites 4.83 and 5.09 ms, 256x256
+// with 4,096 sites 6.05 and 6.23 ms, but with 8,192 sites 8.21 and 7.04 ms (16 SMs do the work
+// of all).
+constexpr uint32_t kChainSites = 4096;
 cudaError_t prepare_site_chain();
 void launch_site_chain(const uint32_t* c0, const uint32_t* c1, Site* sites, float* adam, long long* fix12,
                        uint32_t* nbr, float* raw, const uint32_t* alive, float* tau_a, float* tau_b, SiteGeom* geom,
