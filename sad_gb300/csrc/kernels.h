@@ -338,6 +338,10 @@ void launch_hilbert_pairs(const Site* sites, uint32_t* pairs, uint32_t n, uint32
                           int h, int bits, cudaStream_t st);
 void launch_hilbert_order(const uint32_t* pairs, uint32_t* order, uint32_t* pos, uint32_t n,
                           cudaStream_t st);
+// Both of the above, with what lies between: the Hilbert order and positions of n sites.  pairs
+// holds padded pairs (at least n), sort_temp radix_sort_temp_bytes(padded).
+void launch_hilbert_build(const Site* sites, uint32_t* pairs, uint32_t n, uint32_t padded, int w, int h,
+                          void* sort_temp, uint32_t* order, uint32_t* pos, cudaStream_t st);
 void launch_mse(const float* ren, const float* tgt, const float* mask, float* acc, int w, int h,
                 cudaStream_t st);
 // reproducible form: fixed-point (2^-24) sum into *acc

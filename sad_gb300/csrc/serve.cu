@@ -101,12 +101,8 @@ static sad_status_t render_from_sites_impl(const sad_render_config_t* cfg, const
     launch_pack_geom(sites, r.vgeom, n, st);
     bool use_h = cfg->cand_hilbert_probes > 0 && cfg->cand_hilbert_window > 0;
     if (use_h) {
-        int bits = sad_hilbert_bits_for_size(width, height);
         uint32_t padded = (n + 1023u) / 1024u * 1024u;
-        launch_hilbert_pairs(sites, r.hpairs, n, padded, width, height, bits, st);
-        uint32_t maxk = bits >= 16 ? 0xFFFFFFFFu : (1u << (2 * bits));
-        launch_radix_sort(r.hpairs, padded, maxk, r.sort_temp, st);
-        launch_hilbert_order(r.hpairs, r.horder, r.hpos, n, st);
+        launch_hilbert_build(sites, r.hpairs, n, padded, width, height, r.sort_temp, r.horder, r.hpos, st);
     }
     // the timed candidate build starts here, where the reference starts it: after the
     // per-site preparation, the packed copy and the Hilbert order (sad_cuda.cu:1760-1786)

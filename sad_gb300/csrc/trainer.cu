@@ -111,13 +111,9 @@ static void make_plan(sad_trainer* t) {
 }
 
 static sad_status_t build_hilbert(sad_trainer* t, cudaStream_t s) {
-    int bits = sad_hilbert_bits_for_size(t->w, t->h);
     uint32_t padded = (t->n + 1023u) / 1024u * 1024u;
     padded = std::min(padded, std::max(1u, t->hpadded));
-    launch_hilbert_pairs(t->sites, t->hpairs, t->n, padded, t->w, t->h, bits, s);
-    uint32_t maxk = bits >= 16 ? 0xFFFFFFFFu : (1u << (2 * bits));
-    launch_radix_sort(t->hpairs, padded, maxk, t->sort_temp, s);
-    launch_hilbert_order(t->hpairs, t->horder, t->hpos, t->n, s);
+    launch_hilbert_build(t->sites, t->hpairs, t->n, padded, t->w, t->h, t->sort_temp, t->horder, t->hpos, s);
     t->hilbert_ready = true;
     t->hilbert_count = t->n;
     return check_launch("trainer hilbert order");

@@ -133,6 +133,36 @@ def test_render_from_sites_matches_oracle_pipeline(cuda, orc, w, h, n):
     assert diff.mean() < 2e-4 and np.percentile(diff, 99.9) < 1e-2, (diff.mean(), diff.max())
 
 
+@pytest.mark.parametrize("w,h", [(64, 48), (600, 90)])
+@pytest.mark.parametrize("n", [31, 33, 2047, 2049, 8192, 8193])
+def test_render_from_sites_hilbert_order_is_the_sort_s(cuda, orc, w, h, n):
+    """Order and positions as the render leaves them in its scratch are the stable sort's, with
+    keys that repeat, inactive sites and positions off the image, for lists that are counted
+    into place and lists that are sorted."""
+    from sad_gb300 import _lib
+    sites = cases.scene(w, h, n, 5)[1]
+    rng = np.random.default_rng(n)
+    sites[:, :2] = np.floor(sites[:, :2] / 4) * 4
+    sites[rng.integers(0, n, n // 8), 0] = -1
+    sites[rng.integers(0, n, n // 8), 1] = 2.0 * h
+    cfg = _lib.RenderConfig()
+    _lib.load().sad_render_config_default(cfg)
+    cfg.candidate_passes = 1
+    nbytes = _lib.fn("sad_render_scratch_bytes")(n, w, h, 1)
+    scratch = torch.zeros(nbytes, dtype=torch.uint8, device="cuda")
+    out = torch.empty((h, w, 3), dtype=torch.float32, device="cuda")
+    st = torch.from_numpy(sites).cuda()
+    _lib.call("sad_render_from_sites", C.byref(cfg), C.c_void_p(st.data_ptr()), n, w, h,
+              C.c_void_p(out.data_ptr()), C.c_void_p(scratch.data_ptr()), nbytes, None)
+    torch.cuda.synchronize()
+    bits = orc.hilbert_bits_for_size(w, h)
+    pairs = orc.hilbert_pairs(sites, (n + 1023) // 1024 * 1024, w, h, bits)
+    order, pos = orc.hilbert_order(orc.radix_sort_pairs(pairs, 1 << (2 * bits)), n)
+    left = scratch.cpu().numpy().tobytes()
+    assert np.ascontiguousarray(order, np.uint32).tobytes() in left
+    assert np.ascontiguousarray(pos, np.uint32).tobytes() in left
+
+
 def _tuned_fit(img, cfg, chunks=None):
     from sad_gb300.trainer import Trainer
     h, w = img.shape[:2]
