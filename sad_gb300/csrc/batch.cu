@@ -381,6 +381,8 @@ extern "C" sad_status_t sad_batch_init(sad_batch_t* b) {
     drop_batch_graphs(b);
     b->crowd_end = 0;
     for (sad_trainer* t : b->tr) b->crowd_end = std::max(b->crowd_end, t->crowd_end);
+    // a fit that leaves the batch (sad_trainer_run) reads fields that the batch registered
+    for (sad_trainer* t : b->tr) t->crowd_end = b->crowd_end;
     SAD_TRY(build_tables(b));
     SAD_TRY(check_cuda(cudaStreamSynchronize(b->st), "sad_batch_init: sync"));
     b->iter = 0;

@@ -80,7 +80,8 @@ static void make_plan(sad_trainer* t) {
     int active = t->active;
     uint32_t n = t->n;
     const int freq = c.cand_update_freq;
-    t->crowd_end = freq > 0 ? kCrowdedRefreshes * freq : c.iterations + 1;  // without refreshes: always
+    // always, without refreshes or with few
+    t->crowd_end = freq > 0 && freq <= c.iterations / kCrowdedRefreshes ? kCrowdedRefreshes * freq : c.iterations + 1;
     for (int it = 0; it < c.iterations; ++it) {
         IterPlan& p = t->plan[it];
         if (freq > 0 && it % freq == 0 && active > kCrowdedDensity * (static_cast<double>(t->w) * t->h))

@@ -109,6 +109,6 @@ int refresh_target_field(int passes, int src);
 sad_status_t trainer_build_hilbert(sad_trainer* t, cudaStream_t s);
 // Where iteration `it` stands: 0, its refresh may mark tiles as crowded; 1, not any more, but
 // its gradients may still read a field that has such tiles; 2, neither.
-inline int crowd_stage(int crowd_end, int freq, int it) { return it < crowd_end ? 0 : it < crowd_end + freq ? 1 : 2; }
+inline int crowd_stage(int crowd_end, int freq, int it) { return it < crowd_end ? 0 : it - freq < crowd_end ? 1 : 2; }
 VptParams trainer_vpt_params(sad_trainer* t);
 }  // namespace sad

@@ -52,6 +52,26 @@ def test_batch_matches_single_fits_bitwise(cuda, graphs):
         assert (want_sites[:, 0] >= 0).sum() < CFG["n_sites"]  # the prune events ran
 
 
+@pytest.mark.parametrize("end", [75, 100])
+def test_fit_that_leaves_the_batch(cuda, end):
+    """One image of the batch has a site on most pixels, so the batch marks crowded tiles for
+    longer than a fit of another image alone does (whose tiles still name enough sites for it);
+    each image's fit, continued by its own trainer, ends where a fit alone does."""
+    from sad_gb300.batch import Batch
+    sizes = [(56, 56), (64, 65)]  # 3,000 sites: 0.96 and 0.72 per pixel
+    imgs = [synthetic_image(w, h, seed=7 + i) for i, (w, h) in enumerate(sizes)]
+    with Batch(sizes, use_graphs=1, **CFG) as b:
+        for i, img in enumerate(imgs):
+            b.set_target(i, img)
+        b.init()
+        b.run(end)
+        for t in b.images:
+            t.run()
+        got = [t.sites(active_only=False) for t in b.images]
+    for img, sites in zip(imgs, got):
+        np.testing.assert_array_equal(sites.view(np.uint32), _solo(img, use_graphs=1, **CFG)[0].view(np.uint32))
+
+
 def test_batch_of_more_images_than_one_launch_takes(cuda):
     """The per-pixel stages take their images as kernel parameters, up to 96 per launch;
     a larger batch runs each such stage as several launches, with the same results."""
