@@ -263,10 +263,13 @@ __global__ void __launch_bounds__(256, 4)
         pixel_forward<kRemoval, kSSIM>(prm, x, y, ux, uy, inv_s2, inv_scale, ids, tgt,
                                        [&](int i, SiteGeom& g, float3& c) { src.load(ids[i], g, c); },
                                        wts, rem, valid, pred, dLdp, &finite);
-        // a weight that underflowed adds only zeros, unless its logit is not finite
+        // a weight that underflowed adds only zeros, unless its logit or what it multiplies is
+        // not finite
+        const bool zeros = zero_weight_adds_zeros(dLdp, pred);
 #pragma unroll
         for (int i = 0; i < kCand; ++i)
-            if (!(valid >> i & 1u) || (wts[i] == 0.0f && rem[i] == 0.0f && (finite >> i & 1u))) ids[i] = kEmpty;
+            if (!(valid >> i & 1u) || (zeros && wts[i] == 0.0f && rem[i] == 0.0f && (finite >> i & 1u)))
+                ids[i] = kEmpty;
     }
     const auto load = [=](uint32_t id, SiteGeom& g, float3& c) {
         src.load(id, g, c);

@@ -267,10 +267,12 @@ __global__ void __launch_bounds__(256, 4) render_backward_kernel(
             dLdp = make_float3(__ldg(grad_rgb + 3 * p), __ldg(grad_rgb + 3 * p + 1),
                                __ldg(grad_rgb + 3 * p + 2));
         }
-        // a weight that underflowed adds only zeros, unless its logit is not finite
+        // a weight that underflowed adds only zeros, unless its logit or what it multiplies is
+        // not finite
+        const bool zeros = zero_weight_adds_zeros(dLdp, pred);
 #pragma unroll
         for (int i = 0; i < kCand; ++i)
-            if (!(valid >> i & 1u) || (wts[i] == 0.0f && logits[i] > -INFINITY)) ids[i] = kEmpty;
+            if (!(valid >> i & 1u) || (zeros && wts[i] == 0.0f && logits[i] > -INFINITY)) ids[i] = kEmpty;
     }
     float rem[kCand];
     const auto load = [=](uint32_t id, SiteGeom& g, float3& c) { src.load(id, g, c); };

@@ -77,6 +77,11 @@ __device__ __forceinline__ void folded_range(uint32_t lane, int& first, int& cou
     count = max(0, min(hi - lo, size));
 }
 
+// Whether a zero weight's terms at this pixel are zeros (an infinity or NaN makes them NaN).
+__device__ __forceinline__ bool zero_weight_adds_zeros(float3 dLdp, float3 pred) {
+    return 0.0f * dLdp.x + 0.0f * dLdp.y + 0.0f * dLdp.z + 0.0f * pred.x + 0.0f * pred.y + 0.0f * pred.z == 0.0f;
+}
+
 // What one (pixel, site) adds to the site's sums, in the order of its parameters (position,
 // log_tau, radius, colour, direction, log_aniso): candidate_grads without the factors that
 // sum_scale() holds.

@@ -346,6 +346,32 @@ def test_fused_gradients_match_oracle(ops, orc, w, h, n, removal, masked, ssim):
         assert np.all(np.abs(r - rem) <= 1e-3 * np.maximum(np.abs(rem), 1.0) + 1e-4)
 
 
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_gradients_of_a_pixel_that_is_not_finite(ops, value):
+    """It reaches every active site of the pixel's list, those whose weight is zero too, and no
+    other site."""
+    w, h, n, at = 32, 24, 60, 5 * 32 + 9
+    img, sites = cases.scene(w, h, n, 3)
+    sites[::9, 0] = -1
+    sites[:, 2] = 12.0  # sharp: most weights underflow
+    c0, c1 = cases.random_field(w, h, n, n)
+    ids = np.concatenate([c0[at], c1[at]])
+    listed = np.zeros(n, bool)
+    listed[ids[ids < n]] = True
+    listed &= sites[:, 0] >= 0
+    inv = 1.0 / max(w, h) ** 2
+    gout = np.random.default_rng(2).normal(size=(h, w, 3)).astype(np.float32)
+    gout.reshape(-1, 3)[at] = value
+    got = ops.render_sad_backward(t32(c0), t32(c1), tf(sites), tf(gout), inv, w, h).cpu().numpy()
+    np.testing.assert_array_equal(~np.isfinite(got[:, 4:7]).all(1), listed)
+    img.reshape(-1, 3)[at] = value
+    bufs = _grad_buffers(n)
+    ops.compute_gradients_tiled(t32(c0), t32(c1), tf(img), tf(np.zeros_like(img)),
+                                torch.ones(h, w, device="cuda"), tf(sites), *bufs, inv, 0, 0, 0.0, w, h)
+    got = np.stack([b.cpu().numpy() for b in bufs[4:7]])
+    np.testing.assert_array_equal(~np.isfinite(got).all(0), listed)
+
+
 @pytest.mark.parametrize("w,h,n,removal,ssim", [(1, 1, 9, True, 0.0), (3, 2, 9, False, 0.2), (33, 9, 40, True, 0.0),
                                                 (31, 41, 200, True, 0.2), (5, 64, 64, False, 0.0)])
 def test_fused_gradients_at_patch_edges(ops, orc, w, h, n, removal, ssim):
