@@ -224,8 +224,8 @@ __device__ __forceinline__ void candidate_values(const SiteGeom& g, float3 col, 
 // warp, which sums its sites' gradients by itself (warp_sums.cuh).  Bound by issue.  A torch
 // step (render, gradients, tau diffusion, Adam, candidate refresh) at 768x512 with 24,576
 // sites takes 181 us, 276 us with a key table and float adds in shared memory; at 1237x941
-// with SSIM and removal deltas 332 instead of 555 us.  Four blocks per SM (64 registers):
-// three take 197 and 338 us.
+// with SSIM and removal deltas 318 instead of 575 us.  Four blocks per SM (64 registers): with
+// three or five the latter takes 322 us.
 template <class Src, bool kRemoval, bool kSSIM>
 __global__ void __launch_bounds__(256, 4)
     fused_gradients_kernel(const __grid_constant__ GradParams prm, Src src) {

@@ -10,8 +10,7 @@
 // What is the same for every pixel of a site (softness, scales) is multiplied in after the
 // sum.  Groups of 8 balance the site loop's length, which falls with the group (fewer
 // distinct sites, fewer idle lanes), against the global reductions, which rise: a 1999x1503
-// render and its adjoint took 431 us, with groups of 4, 16 and 32 lanes 450, 448 and 471 us
-// (from raw sites and without the table).
+// render and its adjoint take 372 us, with groups of 4 and 16 lanes 481 and 468 us.
 // A lane sorts its list by id first (19 exchanges), so that the loop compares and shifts its
 // head instead of scanning eight ids for the minimum and for each match (some 20 of 150
 // instructions a round): 372 instead of 394 us there from site records; step at 1237x941 with
