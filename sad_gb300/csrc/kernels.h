@@ -274,7 +274,6 @@ void launch_prune_pairs_batch(const SiteBatchItem* items, const uint32_t* site_p
 void launch_prune_sorted_batch(const SiteBatchItem* items, uint32_t n_items, uint32_t max_k, cudaStream_t st);
 // compaction of every image's [0, n) (max_blocks = the largest compact_blocks(n) of the batch)
 void launch_compact_batch(const SiteBatchItem* items, uint32_t n_items, uint32_t max_blocks, cudaStream_t st);
-void launch_clear_f32(float* buf, size_t count, cudaStream_t st);
 // iteration counter, VPT pass counter and the next iteration's Adam bias corrections
 void launch_reset_state(DevState* state, float beta1, float beta2, cudaStream_t st);
 // Set the tile-table shape rule read by the next tile registrations.

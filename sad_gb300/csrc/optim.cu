@@ -485,19 +485,6 @@ void launch_adam_train(Site* sites, float* adam, long long* fix12, const uint32_
 // ---------------------------------------------------------------------------
 // clears and the iteration counter
 // ---------------------------------------------------------------------------
-__global__ void clear_f32_kernel(float* __restrict__ buf, size_t count) {
-    size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
-    size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
-    for (; i < count; i += stride) buf[i] = 0.0f;
-}
-
-void launch_clear_f32(float* buf, size_t count, cudaStream_t st) {
-    if (count == 0) return;
-    unsigned blocks = static_cast<unsigned>(std::min<size_t>((count + 255) / 256, 152 * 16));
-    clear_f32_kernel<<<blocks, 256, 0, st>>>(buf, count);
-    note_launches(1);
-}
-
 __global__ void clear10_kernel(SoaGrads g, uint32_t n) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -797,6 +784,7 @@ extern "C" sad_status_t sad_clear_gradients(float* g0, float* g1, float* g2, flo
 extern "C" sad_status_t sad_clear_buffer(float* buffer, uint32_t count, sad_stream_t stream) {
     clear_error();
     SAD_REQUIRE(count == 0 || buffer, "sad_clear_buffer: null buffer");
-    launch_clear_f32(buffer, count, as_stream(stream));
-    return check_launch("sad_clear_buffer");
+    if (count == 0) return SAD_OK;
+    return check_cuda(cudaMemsetAsync(buffer, 0, static_cast<size_t>(count) * sizeof(float), as_stream(stream)),
+                      "sad_clear_buffer");
 }
