@@ -359,7 +359,9 @@ struct TermWords {
         for (int k = 0; k < NV; ++k) {
             int h, l;
             split_fix(v[k], h, l);
-            w[warp][lane][k] = static_cast<long long>(h) * (1ll << kSplitLoBits) + l;
+            const long long x = static_cast<long long>(h) * (1ll << kSplitLoBits) + l;
+            // a term past the split's range, which the 64-bit sums still hold, converts in full
+            w[warp][lane][k] = fabsf(v[k]) < 134217728.0f ? x : to_fix(v[k]);
         }
     }
     // all lanes of the warp; adds: the lane has put its words, for site id

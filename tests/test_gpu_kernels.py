@@ -461,6 +461,26 @@ def test_trainer_gradients_match_oracle(ops, orc, w, h, n, field, removal, maske
         assert not fix[:, 10:].any()
 
 
+@pytest.mark.parametrize("target", [-5.0e11, 4.0e11])
+def test_trainer_gradients_of_large_terms(cuda, orc, target):
+    """Terms from 2^27, where a split in two 32-bit words ends, to 2^38, which the 64-bit sums
+    hold: a tile of 2,000 sites (no table holds its keys) with one live pixel, so each sum is
+    one term.  FP32 terms of a random list against FP64: within 1e-3 of the parameter's largest."""
+    w, h, n, at = 16, 16, 2000, 5 * 16 + 7
+    img, sites = cases.scene(w, h, n, 50)
+    sites[:, 2] = 1.0  # soft: every candidate has a weight
+    c0, c1 = cases.random_field(w, h, n, 51, empty_frac=0.0, dup_frac=0.0, invalid_frac=0.0)
+    mask = np.zeros((h, w), np.float32)
+    mask.reshape(-1)[at] = 1.0
+    img.reshape(-1, 3)[at] = target
+    want = orc.compute_gradients_d(c0, c1, img, sites, w, h, mask)
+    largest = np.abs(want).max(axis=1)
+    assert (largest > 2.0 ** 27).sum() >= 6 and largest.max() < 2.0 ** 38
+    fix, _ = _fixed_gradients(w, h, n, c0, c1, img, np.zeros_like(img), mask, sites, False, 0.0)
+    got = fix[:, :10].T / 2.0 ** 24
+    assert (np.abs(got - want) <= 1e-3 * largest[:, None]).all()
+
+
 def test_tau_diffuse_matches_oracle(ops, orc):
     w, h, n = 64, 48, 700
     img, sites = cases.scene(w, h, n, 30)
