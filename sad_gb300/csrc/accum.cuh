@@ -31,8 +31,9 @@ namespace sad {
 constexpr int kFixFracBits = 24;
 constexpr float kFixScale = 16777216.0f;                  // 2^24
 constexpr float kFixInvScale = 5.9604644775390625e-08f;  // 2^-24
-// The log_tau word of an inactive site's record (which no gradient is added to): the tau passes
-// read a neighbour's gradient and whether it is active in one gather.
+// The log_tau word of a record that no gradient is added to (position.x < 0): the tau passes read
+// a neighbour's gradient and whether it is active in one gather.  An active site's sum can be
+// the same word (to_fix of a NaN, or of anything from -2^39 down).
 constexpr long long kInactiveWord = -0x7fffffffffffffffll - 1;
 constexpr int kTauWord = 2;
 // Per tile, a fixed-point sum is kept as two 32-bit words (hi * 2^20 + lo): shared

@@ -200,7 +200,7 @@ void launch_tau_diffuse_raw(const uint32_t* c0, const uint32_t* c1, const Site* 
 void launch_tau_first_pass(const uint32_t* c0, const uint32_t* c1, const SiteGeom* geom,
                            const long long* fix12, uint32_t* nbr, float* raw, const uint32_t* alive,
                            float* gout, uint32_t n, uint32_t max_alive, const DevState* state,
-                           int iterations, int w, int h, int ds, cudaStream_t st);
+                           int iterations, int w, int h, int ds, bool by_position, cudaStream_t st);
 // trainer form, middle passes from the recorded lists
 void launch_tau_list_pass(const uint32_t* nbr, const float* raw, const uint32_t* alive,
                           const float* gin, float* gout, uint32_t max_alive, const DevState* state,
@@ -229,7 +229,8 @@ cudaError_t prepare_site_chain();
 void launch_site_chain(const uint32_t* c0, const uint32_t* c1, Site* sites, float* adam, long long* fix12,
                        uint32_t* nbr, float* raw, const uint32_t* alive, float* tau_a, float* tau_b, SiteGeom* geom,
                        SiteColor* color, const AdamHyper& hp, DevState* state, int iterations, uint32_t n, int cw,
-                       int ch, int ds, int w, int h, bool advance, uint32_t vpt_passes, cudaStream_t st);
+                       int ch, int ds, int w, int h, bool by_position, bool advance, uint32_t vpt_passes,
+                       cudaStream_t st);
 // Batched per-site launches over the compacted active lists of every image of a batch,
 // walked as one flat list: site_prefix[i] = sum of the n_alive of images < i (in device
 // memory, written by launch_batch_site_prefix after each compaction); grid-stride, so the

@@ -82,7 +82,8 @@ __device__ __forceinline__ float tau_lambda(uint32_t iter, int iterations) {
 // float; the middle passes read the list; the last pass runs inside the Adam kernel.
 // Every pass walks the compacted list of active sites (state->n_alive entries): an
 // inactive site's diffused value is never read (a neighbour must be active, and Adam
-// skips inactive sites).
+// skips inactive sites).  by_position: some sites have position.x NaN, which makes them
+// neither active nor, to the gradient kernel and the candidate passes, inactive.
 struct TauLists {
     uint4* nbr;            // [n][2] neighbour ids, kEmpty-padded
     float* raw;            // [n] raw log-tau gradient (float)
@@ -93,20 +94,20 @@ __device__ __forceinline__ void tau_first_one(const uint4* __restrict__ c0, cons
                                               const SiteGeom* __restrict__ geom,
                                               const long long* __restrict__ fix12, const TauLists& tl,
                                               float* __restrict__ gout, uint32_t n, uint32_t i,
-                                              float lambda, int w, int h, int ds);
+                                              float lambda, int w, int h, int ds, bool by_position);
 
 __global__ void tau_first_pass_kernel(const uint4* __restrict__ c0, const uint4* __restrict__ c1,
                                       const SiteGeom* __restrict__ geom,
                                       const long long* __restrict__ fix12, TauLists tl,
                                       float* __restrict__ gout, uint32_t n,
                                       const DevState* __restrict__ state, int iterations, int w,
-                                      int h, int ds) {
+                                      int h, int ds, bool by_position) {
     pdl_wait();
     const uint32_t n_alive = state->n_alive;
     const float lambda = tau_lambda(state->iter, iterations);
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n_alive; j += gridDim.x * blockDim.x) {
         const uint32_t i = tl.alive[j];
-        tau_first_one(c0, c1, geom, fix12, tl, gout, n, i, lambda, w, h, ds);
+        tau_first_one(c0, c1, geom, fix12, tl, gout, n, i, lambda, w, h, ds, by_position);
     }
 }
 
@@ -114,7 +115,7 @@ __device__ __forceinline__ void tau_first_one(const uint4* __restrict__ c0, cons
                                               const SiteGeom* __restrict__ geom,
                                               const long long* __restrict__ fix12, const TauLists& tl,
                                               float* __restrict__ gout, uint32_t n, uint32_t i,
-                                              float lambda, int w, int h, int ds) {
+                                              float lambda, int w, int h, int ds, bool by_position) {
     float2 sp = __ldg(reinterpret_cast<const float2*>(geom + i));
     const float r = from_fix(fix12[static_cast<size_t>(i) * 12 + kTauWord]);
     tl.raw[i] = r;
@@ -126,7 +127,9 @@ __device__ __forceinline__ void tau_first_one(const uint4* __restrict__ c0, cons
     uint32_t ids[kCand] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
     // every candidate's raw gradient is fetched before any is used, so the gathers overlap
     // instead of forming a chain of dependent loads; an inactive site's word says so (with its
-    // position gathered too, the pass over a 6-image batch's 768,000 sites took 66 us)
+    // position gathered too, the pass over a 6-image batch's 768,000 sites took 66 us).  The
+    // word alone does not: the sum of an active site can come to it (a NaN or infinite term
+    // does), so the position decides for the few that carry it.
     long long cfix[kCand];
 #pragma unroll
     for (int k = 0; k < kCand; ++k) {
@@ -141,6 +144,7 @@ __device__ __forceinline__ void tau_first_one(const uint4* __restrict__ c0, cons
         list[k] = kEmpty;
         uint32_t m = ids[k];
         bool take = cfix[k] != kInactiveWord;
+        if (by_position || !take) take = m < n && m != i && __ldg(&geom[m].px) >= 0.0f;
 #pragma unroll
         for (int j = 0; j < k; ++j) take &= ids[j] != m;
         if (take) {
@@ -195,12 +199,12 @@ __global__ void tau_list_pass_kernel(TauLists tl, const float* __restrict__ gin,
 void launch_tau_first_pass(const uint32_t* c0, const uint32_t* c1, const SiteGeom* geom,
                            const long long* fix12, uint32_t* nbr, float* raw, const uint32_t* alive,
                            float* gout, uint32_t n, uint32_t max_alive, const DevState* state,
-                           int iterations, int w, int h, int ds, cudaStream_t st) {
+                           int iterations, int w, int h, int ds, bool by_position, cudaStream_t st) {
     if (max_alive == 0) return;
     TauLists tl{reinterpret_cast<uint4*>(nbr), raw, alive};
     launch_pdl(tau_first_pass_kernel, dim3(blocks_for(max_alive, 256)), dim3(256), 0, st,
                reinterpret_cast<const uint4*>(c0), reinterpret_cast<const uint4*>(c1), geom, fix12, tl, gout, n,
-               state, iterations, w, h, ds);
+               state, iterations, w, h, ds, by_position);
     note_launches(1);
 }
 
@@ -539,14 +543,15 @@ __global__ void __launch_bounds__(kChainThreads)
     site_chain_kernel(const uint4* __restrict__ c0, const uint4* __restrict__ c1, Site* sites, float* adam,
                       long long* fix12, TauLists tl, float* tau_a, float* tau_b, SiteGeom* geom, SiteColor* color,
                       AdamHyper hp, DevState* state, int iterations, uint32_t n, int cw, int ch, int ds, int w, int h,
-                      bool advance, uint32_t vpt_passes) {
+                      bool by_position, bool advance, uint32_t vpt_passes) {
     extern __shared__ __align__(16) unsigned char sad_chain_smem[];
     pdl_wait();
     const uint32_t n_alive = state->n_alive;
     const StepScalars step = step_scalars(state, iterations);
     const uint32_t first = blockIdx.x * kChainThreads + threadIdx.x, stride = kChainBlocks * kChainThreads;
     for (uint32_t j = first; j < n_alive; j += stride)
-        tau_first_one(c0, c1, geom, fix12, tl, tau_a, n, tl.alive[j], step.lambda, cw, ch, ds);
+        tau_first_one(c0, c1, geom, fix12, tl, tau_a, n, tl.alive[j], step.lambda, cw, ch, ds,
+                      by_position);
     cluster_barrier();
     if (advance && first == 0) {  // every block has read the state
         state->iter += 1u;
@@ -581,7 +586,8 @@ cudaError_t prepare_site_chain() {
 void launch_site_chain(const uint32_t* c0, const uint32_t* c1, Site* sites, float* adam, long long* fix12,
                        uint32_t* nbr, float* raw, const uint32_t* alive, float* tau_a, float* tau_b, SiteGeom* geom,
                        SiteColor* color, const AdamHyper& hp, DevState* state, int iterations, uint32_t n, int cw,
-                       int ch, int ds, int w, int h, bool advance, uint32_t vpt_passes, cudaStream_t st) {
+                       int ch, int ds, int w, int h, bool by_position, bool advance, uint32_t vpt_passes,
+                       cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kChainBlocks);
     cfg.blockDim = dim3(kChainThreads);
@@ -598,7 +604,7 @@ void launch_site_chain(const uint32_t* c0, const uint32_t* c1, Site* sites, floa
     TauLists tl{reinterpret_cast<uint4*>(nbr), raw, alive};
     cudaLaunchKernelEx(&cfg, site_chain_kernel, reinterpret_cast<const uint4*>(c0), reinterpret_cast<const uint4*>(c1),
                        sites, adam, fix12, tl, tau_a, tau_b, geom, color, hp, state, iterations, n, cw, ch, ds, w, h,
-                       advance, vpt_passes);
+                       by_position, advance, vpt_passes);
     note_launches(1);
 }
 
@@ -641,7 +647,7 @@ __global__ void __launch_bounds__(256) tau_first_batch_kernel(const SiteBatchIte
         const uint32_t i = it.alive[g - s_prefix[k]];
         tau_first_one(reinterpret_cast<const uint4*>(it.cand0[field]), reinterpret_cast<const uint4*>(it.cand1[field]),
                       it.geom, it.grads, tl, it.tau_a, it.n, i, tau_lambda(it.state->iter, iterations), it.cw,
-                      it.ch, it.ds);
+                      it.ch, it.ds, false);
     }
 }
 

@@ -206,10 +206,10 @@ __global__ void prune_sorted_kernel(Site* __restrict__ sites, SiteGeom* __restri
     fix12[static_cast<size_t>(s) * 12 + kTauWord] = kInactiveWord;
 }
 
-// Marks the gradient records of the sites that are not active.
+// Marks the gradient records of the sites that no gradient is added to (accum.cuh).
 __global__ void mark_inactive_kernel(const Site* __restrict__ sites, long long* __restrict__ fix12, uint32_t n) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && !(sites[i].px >= 0.0f)) fix12[static_cast<size_t>(i) * 12 + kTauWord] = kInactiveWord;
+    if (i < n && sites[i].px < 0.0f) fix12[static_cast<size_t>(i) * 12 + kTauWord] = kInactiveWord;
 }
 
 void launch_mark_inactive(const Site* sites, long long* fix12, uint32_t n, cudaStream_t st) {

@@ -257,12 +257,13 @@ static int iteration_body(sad_trainer* t, bool upd, bool prune, int field, int a
         if (chain) {
             launch_site_chain(t->cand0[next], t->cand1[next], t->sites, t->adam, t->grads, t->tau_nbr, t->tau_raw,
                               t->alive, t->tau_a, t->tau_b, t->geom, t->color, hp, t->state, t->cfg.iterations, t->n,
-                              t->cw, t->ch, t->ds, t->w, t->h, !prune, static_cast<uint32_t>(adv_passes), s);
+                              t->cw, t->ch, t->ds, t->w, t->h, t->nan_positions, !prune,
+                              static_cast<uint32_t>(adv_passes), s);
             if (!prune) return next;  // the state is advanced too
         } else {
             launch_tau_first_pass(t->cand0[next], t->cand1[next], t->geom, t->grads, t->tau_nbr, t->tau_raw,
                                   t->alive, t->tau_a, t->n, hint, t->state, t->cfg.iterations, t->cw, t->ch,
-                                  t->ds, s);
+                                  t->ds, t->nan_positions, s);
             launch_tau_list_pass(t->tau_nbr, t->tau_raw, t->alive, t->tau_a, t->tau_b, hint, t->state,
                                  t->cfg.iterations, s);
             launch_tau_list_pass(t->tau_nbr, t->tau_raw, t->alive, t->tau_b, t->tau_a, hint, t->state,
@@ -631,6 +632,7 @@ extern "C" sad_status_t sad_trainer_init(sad_trainer_t* t, const float* sites_ho
     cudaStream_t s = t->st;
     uint32_t n0;
     int active;
+    t->nan_positions = false;
     if (sites_host) {
         SAD_REQUIRE(n > 0 && static_cast<uint32_t>(n) <= t->cap, "sad_trainer_init: site count exceeds capacity");
         n0 = static_cast<uint32_t>(n);
@@ -638,7 +640,11 @@ extern "C" sad_status_t sad_trainer_init(sad_trainer_t* t, const float* sites_ho
                                            cudaMemcpyHostToDevice, s),
                            "trainer sites upload"));
         active = 0;
-        for (int i = 0; i < n; ++i) active += sites_host[static_cast<size_t>(i) * 10] >= 0.0f;
+        for (int i = 0; i < n; ++i) {
+            const float x = sites_host[static_cast<size_t>(i) * 10];
+            active += x >= 0.0f;
+            t->nan_positions |= x != x;
+        }
     } else {
         n0 = static_cast<uint32_t>(t->cfg.n_sites);
         SAD_REQUIRE(n0 <= t->cap, "sad_trainer_init: n_sites exceeds capacity");

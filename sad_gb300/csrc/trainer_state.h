@@ -38,6 +38,7 @@ struct sad_trainer {
     std::vector<sad::IterPlan> plan;
     int crowd_end = 0;  // refreshes before this iteration may mark tiles as crowded
     int stage = 0;      // crowd_stage() of the iteration being launched
+    bool nan_positions = false;  // sites were uploaded with position.x NaN
 
     float* target = nullptr;
     float* mask = nullptr;

@@ -199,3 +199,65 @@ def test_autotuner_leaves_the_fit_bit_identical(cuda):
     a, _ = _tuned_fit(img, small_cfg(autotune=0, **pruned))
     b, _ = _tuned_fit(img, small_cfg(autotune=1, **pruned))
     np.testing.assert_array_equal(a, b)
+
+
+# One live pixel whose terms saturate: the log_tau sums of its candidates are -2^63 or 2^63 - 1
+# units of 2^-24, which the tau passes spread to the sites that list them.  nan: one of the
+# candidates has position NaN, which puts it 1e-4 from every pixel (fmaxf drops the NaN): it
+# has a weight and a gradient and is in most lists, but is not active and takes no part.
+@pytest.mark.parametrize("n", [4000, 4200])  # one launch for the per-site work, and several
+@pytest.mark.parametrize("nan", [False, True])
+def test_tau_diffusion_of_saturated_gradients(cuda, orc, n, nan):
+    from sad_gb300 import _lib
+    from sad_gb300.trainer import Trainer
+    w, h, at = 16, 16, 5 * 16 + 7
+    img, sites = cases.scene(w, h, n, 60)
+    sites[:, 2] = 1.0
+    sites[::17, 0] = -1.0
+    c0, c1 = orc.init_candidates(n, 0, 0, w, h)
+    if nan:
+        sites[c1[at, 1], 0] = np.nan
+    c0 = orc.jfa_seed(c0, sites, w, h)
+    listed = np.concatenate([c0[at], c1[at]])
+    active = sites[:, 0] >= 0
+    mask = np.zeros((h, w), np.float32)
+    mask.reshape(-1)[at] = 1.0
+    img.reshape(-1, 3)[at] = -1.0e30
+    cfg = small_cfg(n_sites=n, max_sites=n, iterations=1, prune_percentile=0.0, cand_update_freq=4, cand_hilbert_probes=0,
+                    cand_radius_probes=0, lr_pos=0.0, lr_radius=0.0, lr_color=0.0, lr_dir=0.0,
+                    lr_aniso=0.0)
+    nbytes = _lib.fn("sad_trainer_memory_bytes")(C.byref(cfg), w, h)
+    memory = torch.full((nbytes,), 0x7F, dtype=torch.uint8, device="cuda")  # 3.4e38 wherever nothing is written
+    torch.cuda.synchronize()
+    tr = Trainer.__new__(Trainer)
+    tr.width, tr.height, tr.cfg, tr._h = w, h, cfg, C.c_void_p()
+    _lib.call("sad_trainer_create_in", C.byref(cfg), w, h, C.c_void_p(memory.data_ptr()), nbytes, C.byref(tr._h))
+    with tr:
+        tr.set_target(img, mask)
+        tr.init(sites)
+        tr.run()
+        got = tr.sites(active_only=False)[:, 2]
+    s = sites[listed].astype(np.float64)
+    dx, dy, inv = at % w - s[:, 0], at // w - s[:, 1], 1.0 / max(w, h) ** 2
+    proj = s[:, 7] * dx + s[:, 8] * dy
+    l1 = np.exp(s[:, 9])
+    d2 = np.fmax((l1 * proj ** 2 + np.fmax(dx ** 2 + dy ** 2 - proj ** 2, 0) / l1) * inv, 1e-8)
+    dist = np.sqrt(d2) - s[:, 3] * np.sqrt(inv)
+    z = np.where(s[:, 0] < 0, -np.inf, -np.exp(1.0) * dist)
+    wts = np.exp(z - z.max())
+    wts /= wts.sum()
+    pred = (wts[:, None] * s[:, 4:7])[active[listed]].sum(0)
+    term = -(wts[:, None] * 2.0e30 * (s[:, 4:7] - pred)).sum(1) * dist * np.exp(1.0)
+    raw = np.zeros(n, np.float32)
+    raw[listed] = np.where(active[listed], np.sign(term), 0.0) * 2.0 ** 39
+    assert (np.abs(term[active[listed]]) > 2.0 ** 64).all() and (term < 0).any()
+    step = orc.pack_jump_step(0, w, h)
+    c0, c1 = orc.vpt_pass(c0, c1, orc.pack_sites(sites), n, step, 0, w, h, 64.0, 0, cfg.cand_inject_count)
+    sites[np.isnan(sites[:, 0]), 0] = -1.0  # for the diffusion
+    g = raw.copy()
+    for _ in range(4):
+        g = orc.tau_diffuse(c0, c1, sites, raw, g, 0.005, w, h)
+    moved = active & (g != 0)
+    assert moved.sum() > 100  # far more than the pixel's own candidates
+    want = sites[:, 2] - np.where(moved, cfg.lr_tau * np.sign(g), 0.0)  # Adam's first step is its rate
+    np.testing.assert_allclose(got, want, atol=0.01 * cfg.lr_tau)
