@@ -142,7 +142,8 @@ struct MetricTerms {
     float dx, dy;   // uv - position
     float proj;     // dir . diff
     float proj2, perp2;
-    float d2_safe;  // max(normalised anisotropic distance^2, 1e-8)
+    float d2_norm;  // normalised anisotropic distance^2
+    float d2_safe;  // max(d2_norm, 1e-8)
 };
 
 __device__ __forceinline__ MetricTerms metric_terms(const SiteGeom& g, float ux, float uy,
@@ -155,8 +156,8 @@ __device__ __forceinline__ MetricTerms metric_terms(const SiteGeom& g, float ux,
     m.proj2 = m.proj * m.proj;
     m.perp2 = fmaxf(diff2 - m.proj2, 0.0f);
     float d2_aniso = g.l1 * m.proj2 + g.l2 * m.perp2;
-    float d2_norm = d2_aniso * inv_scale_sq;
-    m.d2_safe = fmaxf(d2_norm, 1e-8f);
+    m.d2_norm = d2_aniso * inv_scale_sq;
+    m.d2_safe = fmaxf(m.d2_norm, 1e-8f);
     return m;
 }
 
@@ -165,6 +166,15 @@ __device__ __forceinline__ float dmix2(const SiteGeom& g, float ux, float uy, fl
                                        float inv_scale) {
     MetricTerms m = metric_terms(g, ux, uy, inv_scale_sq);
     return sqrtf(m.d2_safe) - g.radius * inv_scale;
+}
+
+// The logit of a site at a pixel; finite: and neither it nor the distance that fmaxf bounds from
+// below (which drops a NaN) is an infinity or NaN.
+__device__ __forceinline__ float site_logit(const SiteGeom& g, float ux, float uy, float inv_scale_sq,
+                                            float inv_scale, bool& finite) {
+    const float logit = -g.tau * dmix2(g, ux, uy, inv_scale_sq, inv_scale);
+    finite = fabsf(fmaf(0.0f, metric_terms(g, ux, uy, inv_scale_sq).d2_norm, logit)) < INFINITY;
+    return logit;
 }
 
 // Item of flat index g in a batch walked as one list: prefix (shared or global) holds the

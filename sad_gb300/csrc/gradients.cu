@@ -111,7 +111,7 @@ struct GradLayout {
 // with kRemoval, the removal delta on the first slot of each distinct valid site.
 // site(i, g, col) supplies candidate i's data.  Semantics of
 // backends/cuda/src/gradients.cu:103-300.
-// finite (nullable) receives the slots whose logit is finite.
+// finite (nullable) receives the slots whose logit and distance are finite.
 template <bool kRemoval, bool kSSIM, class SiteFn>
 __device__ __forceinline__ void pixel_forward(const GradParams& prm, int x, int y, float ux,
                                               float uy, float inv_s2, float inv_scale,
@@ -134,19 +134,14 @@ __device__ __forceinline__ void pixel_forward(const GradParams& prm, int x, int 
         if (g.px < 0.0f) continue;
         valid |= 1u << i;
         if (g.px >= 0.0f) blend |= 1u << i;
-        float tau = g.tau;
-        float d = dmix2(g, ux, uy, inv_s2, inv_scale);
-        logits[i] = -tau * d;
+        bool whole;
+        logits[i] = site_logit(g, ux, uy, inv_s2, inv_scale, whole);
+        if (finite && whole) *finite |= 1u << i;
         mx = fmaxf(mx, logits[i]);
     }
     if (isinf(mx) && mx < 0.0f) {
         valid = 0;
         return;
-    }
-    if (finite) {
-#pragma unroll
-        for (int i = 0; i < kCand; ++i)
-            if (fabsf(logits[i]) < INFINITY) *finite |= 1u << i;
     }
     float sum = 0.0f;
 #pragma unroll
@@ -263,8 +258,8 @@ __global__ void __launch_bounds__(256, 4)
         pixel_forward<kRemoval, kSSIM>(prm, x, y, ux, uy, inv_s2, inv_scale, ids, tgt,
                                        [&](int i, SiteGeom& g, float3& c) { src.load(ids[i], g, c); },
                                        wts, rem, valid, pred, dLdp, &finite);
-        // a weight that underflowed adds only zeros, unless its logit or what it multiplies is
-        // not finite
+        // a weight that underflowed adds only zeros, unless the site's geometry, its logit or what
+        // the weight multiplies is not finite
         const bool zeros = zero_weight_adds_zeros(dLdp, pred);
 #pragma unroll
         for (int i = 0; i < kCand; ++i)

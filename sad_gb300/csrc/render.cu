@@ -232,6 +232,7 @@ __global__ void __launch_bounds__(256, 4) render_backward_kernel(
         float mx = -INFINITY;
         uint32_t valid = 0;  // softmax members: id < n and !(position.x < 0)
         uint32_t blend = 0;  // colour contributors: position.x >= 0
+        uint32_t finite = 0;  // logit and distance
 #pragma unroll
         for (int i = 0; i < kCand; ++i) {
             logits[i] = -INFINITY;
@@ -242,7 +243,9 @@ __global__ void __launch_bounds__(256, 4) render_backward_kernel(
             if (g.px < 0.0f) continue;
             valid |= 1u << i;
             if (g.px >= 0.0f) blend |= 1u << i;
-            logits[i] = -g.tau * dmix2(g, ux, uy, inv_s2, inv_scale);
+            bool whole;
+            logits[i] = site_logit(g, ux, uy, inv_s2, inv_scale, whole);
+            if (whole) finite |= 1u << i;
             mx = fmaxf(mx, logits[i]);
         }
         // compute_candidate_weights_raw bails out when nothing is valid or max is +-inf
@@ -268,12 +271,12 @@ __global__ void __launch_bounds__(256, 4) render_backward_kernel(
             dLdp = make_float3(__ldg(grad_rgb + 3 * p), __ldg(grad_rgb + 3 * p + 1),
                                __ldg(grad_rgb + 3 * p + 2));
         }
-        // a weight that underflowed adds only zeros, unless its logit or what it multiplies is
-        // not finite
+        // a weight that underflowed adds only zeros, unless the site's geometry, its logit or what
+        // the weight multiplies is not finite
         const bool zeros = zero_weight_adds_zeros(dLdp, pred);
 #pragma unroll
         for (int i = 0; i < kCand; ++i)
-            if (!(valid >> i & 1u) || (zeros && wts[i] == 0.0f && logits[i] > -INFINITY)) ids[i] = kEmpty;
+            if (!(valid >> i & 1u) || (zeros && wts[i] == 0.0f && (finite >> i & 1u))) ids[i] = kEmpty;
     }
     float rem[kCand];
     const auto load = [=](uint32_t id, SiteGeom& g, float3& c) { src.load(id, g, c); };

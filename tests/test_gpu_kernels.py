@@ -372,6 +372,32 @@ def test_gradients_of_a_pixel_that_is_not_finite(ops, value):
     np.testing.assert_array_equal(~np.isfinite(got).all(0), listed)
 
 
+@pytest.mark.parametrize("column", [0, 1, 7, 8, 9])  # position, direction, log_aniso
+def test_gradients_of_a_site_that_is_not_finite(ops, orc, column):
+    """A NaN in its geometry leaves a site's distance finite (fmaxf drops it), 1e-4 from every
+    pixel, and makes its gradients NaN where its weight is zero, too: two such sites, the first
+    of the larger radius and in every list, so that the second's weight is always zero."""
+    w, h, n = 32, 24, 60
+    img, sites = cases.scene(w, h, n, 3)
+    sites[:, 2] = 12.0
+    sites[:2, column], sites[:2, 3] = np.nan, [9.0, 2.0]
+    sites[2:, 3] = 1.0
+    c0, c1 = cases.random_field(w, h, n, n)
+    c0[:, 0] = 0
+    inv = 1.0 / max(w, h) ** 2
+    gout = np.random.default_rng(2).normal(size=(h, w, 3)).astype(np.float32)
+    got = ops.render_sad_backward(t32(c0), t32(c1), tf(sites), tf(gout), inv, w, h).cpu().numpy()
+    want, _ = orc.render_backward(c0, c1, sites, gout, w, h)
+    assert (~np.isfinite(want[1])).any() and np.isfinite(want[2:]).all()
+    np.testing.assert_array_equal(np.isfinite(got), np.isfinite(want))
+    bufs = _grad_buffers(n)
+    ops.compute_gradients_tiled(t32(c0), t32(c1), tf(img), tf(np.zeros_like(img)),
+                                torch.ones(h, w, device="cuda"), tf(sites), *bufs, inv, 0, 0, 0.0, w, h)
+    want, _, _ = orc.compute_gradients(c0, c1, img, sites, w, h)
+    got = np.stack([b.cpu().numpy() for b in bufs[:10]])
+    np.testing.assert_array_equal(np.isfinite(got), np.isfinite(want))
+
+
 @pytest.mark.parametrize("w,h,n,removal,ssim", [(1, 1, 9, True, 0.0), (3, 2, 9, False, 0.2), (33, 9, 40, True, 0.0),
                                                 (31, 41, 200, True, 0.2), (5, 64, 64, False, 0.0)])
 def test_fused_gradients_at_patch_edges(ops, orc, w, h, n, removal, ssim):
