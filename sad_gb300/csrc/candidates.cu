@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(kVptThreads, 5) jfa_flood_kernel(const uint4* 
                                                                   FloodTiling tiling) {
     __shared__ uint32_t s_queue[12 * kVptThreads];  // one row's lists
     pdl_wait();
-    const int2 at = tiling.texel(blockIdx.x, blockIdx.y);
+    const int2 at = tiling.texel(blockIdx.x, blockIdx.z * gridDim.y + blockIdx.y);
     const int x = at.x, y = at.y;
     if (x >= w || y >= h) return;
     VptQueue q = thread_queue(s_queue);
@@ -689,8 +689,13 @@ static FloodTiling flood_tiling(uint32_t step, uint32_t n, int w, int h) {
 template <class Src>
 static void launch_jfa_flood(const uint32_t* in0, uint32_t* out0, Src src, uint32_t n, uint32_t step,
                              float inv_s2, int w, int h, int ds, int tw, int th, cudaStream_t st) {
-    const FloodTiling t = flood_tiling(step, n, w, h);
-    const dim3 grid((w + t.span_x() - 1) / t.span_x() * t.fill_x(), (h + t.span_y() - 1) / t.span_y() * t.fill_y());
+    FloodTiling t = flood_tiling(step, n, w, h);
+    // a block takes four rows at stride 1: past the limit of the grid's y the rows of blocks are
+    // halved into z, so that a field may have 524,280 rows, as with eight a block
+    const auto rows = [&] { return (h + t.span_y() - 1) / t.span_y() * t.fill_y(); };
+    while (t.log2 > 0 && rows() > 2 * kMaxGridRows) --t.log2;
+    const int folds = rows() > kMaxGridRows ? 2 : 1;
+    const dim3 grid((w + t.span_x() - 1) / t.span_x() * t.fill_x(), (rows() + folds - 1) / folds, folds);
     launch_pdl(jfa_flood_kernel<Src>, grid, dim3(32, 8), 0, st, reinterpret_cast<const uint4*>(in0),
                reinterpret_cast<uint4*>(out0), src, n, step, inv_s2, w, h, ds, tw, th, t);
     note_launches(1);

@@ -77,6 +77,9 @@ inline bool image_size_ok(int w, int h) {
     return w > 0 && h > 0 && static_cast<long long>(w) * h <= kMaxPixels;
 }
 
+// The limit of a grid's y and z dimensions.
+constexpr int kMaxGridRows = 65535;
+
 inline unsigned blocks_for(size_t n, unsigned threads) {
     return static_cast<unsigned>((n + threads - 1) / threads);
 }

@@ -60,3 +60,50 @@ def test_render_from_sites_at_degenerate_sizes(cuda, w, h, n):
     # every pixel is written, and is a convex combination of the site colours
     assert np.isfinite(o).all()
     assert o.min() >= 0.2 - 1e-5 and o.max() <= 0.8 + 1e-5
+
+
+def _tall(w, h, n):
+    """Sites down a tall image, with exact FP32 distances (whole pixels, unit softness, no
+    anisotropy; max side 2^18 for the scale)."""
+    rng = np.random.default_rng(h)
+    s = np.zeros((n, 10), np.float32)
+    s[:, 0], s[:, 1] = rng.integers(0, w, n), np.sort(rng.integers(0, h, n))
+    s[:, 3], s[:, 7] = rng.integers(1, 9, n), 1.0
+    s[:, 4:7] = rng.uniform(0.2, 0.8, (n, 3))
+    return s
+
+
+@pytest.mark.parametrize("w,h,step", [(2, 262140, 1), (2, 262141, 1), (1, 300001, 4), (2, 524280, 2),
+                                      (80, 264000, 8)])
+def test_flood_of_tall_fields(cuda, orc, w, h, step):
+    """Rows of blocks on either side of the grid's y limit (four texel rows a block)."""
+    from sad_gb300 import ops
+    sites = _tall(w, h, 5000)
+    rng = np.random.default_rng(w)
+    f = rng.integers(0, 5000, (w * h, 4)).astype(np.uint32)
+    f[(np.arange(w * h) // w) % 3 == 1] = 0xFFFFFFFF
+    near = np.searchsorted(sites[:, 1], np.arange(h)).clip(0, 4999).repeat(w)
+    f[:, 0] = np.where(f[:, 0] == 0xFFFFFFFF, f[:, 0], near)
+    inv = 2.0 ** -36
+    out = torch.full((w * h, 4), -2, dtype=torch.int32, device="cuda")
+    ops.jfa_flood(torch.from_numpy(f.view(np.int32)).cuda(), out, torch.from_numpy(sites).cuda(), inv, 0, step, 1, w, h)
+    want = orc.jfa_flood(f, sites, step, w, h, inv_s2=inv)
+    np.testing.assert_array_equal(out.cpu().numpy().view(np.uint32), want)
+
+
+def test_render_of_a_tall_image(cuda):
+    """A render from sites whose flood has more rows of blocks than the grid's y takes: pixels
+    between 0.2 and 0.8, the range of the sites' colours."""
+    from sad_gb300 import _lib
+    w, h, n = 2, 300000, 3000
+    sites = torch.from_numpy(_tall(w, h, n)).cuda()
+    cfg = _lib.RenderConfig()
+    _lib.fn("sad_render_config_default")(C.byref(cfg))
+    nb = _lib.fn("sad_render_scratch_bytes")(n, w, h, cfg.cand_downscale)
+    scratch = torch.empty(nb, dtype=torch.uint8, device="cuda")
+    out = torch.full((h, w, 3), -1.0, device="cuda")
+    _lib.call("sad_render_from_sites", C.byref(cfg), C.c_void_p(sites.data_ptr()), n, w, h,
+              C.c_void_p(out.data_ptr()), C.c_void_p(scratch.data_ptr()), nb, None)
+    torch.cuda.synchronize()
+    o = out.cpu().numpy()
+    assert o.min() >= 0.2 - 1e-5 and o.max() <= 0.8 + 1e-5
