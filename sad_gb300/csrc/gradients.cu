@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(256, 4)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int2 at = sum_patch_pixel(lane);
     const int x = blockIdx.x * 32 + (warp & 3) * 8 + at.x;
-    const int y = blockIdx.y * 8 + (warp >> 2) * 4 + at.y;
+    const int y = (blockIdx.z * gridDim.y + blockIdx.y) * 8 + (warp >> 2) * 4 + at.y;
     const int w = prm.width, h = prm.height;
     const float inv_s2 = prm.inv_scale_sq;
     const float inv_scale = sqrtf(inv_s2);
@@ -627,7 +627,9 @@ cudaError_t prepare_gradient_kernels() {
 
 template <class Src>
 static void launch_gradients_float(const GradParams& p, Src src, cudaStream_t st) {
-    const dim3 grid((p.width + 31) / 32, (p.height + 7) / 8);
+    // rows of blocks past the limit of the grid's y are halved into z: 1,048,560 rows, as with 16 a block
+    const int rows = (p.height + 7) / 8, folds = rows > kMaxGridRows ? 2 : 1;
+    const dim3 grid((p.width + 31) / 32, (rows + folds - 1) / folds, folds);
     with_constant(p.compute_removal != 0, [&](auto removal) {
         with_constant(p.ssim_weight > 0.0f, [&](auto ssim) {
             fused_gradients_kernel<Src, removal, ssim><<<grid, 256, 0, st>>>(p, src);

@@ -91,6 +91,29 @@ def test_flood_of_tall_fields(cuda, orc, w, h, step):
     np.testing.assert_array_equal(out.cpu().numpy().view(np.uint32), want)
 
 
+@pytest.mark.parametrize("w,h", [(1, 524280), (1, 524281), (2, 600000), (1, 1048560)])
+def test_gradients_of_tall_images(cuda, orc, w, h):
+    """Rows of blocks on either side of the grid's y limit (eight pixel rows a block), every pixel
+    with the sites around it, against the FP64 sums (the FP32 oracle's texel of a pixel overflows
+    above 46,340 rows).  FP32 terms with exact distances and some 1,000 of them a site: 1e-3 of
+    each parameter's norm allows for sums that cancel to a thousandth."""
+    from sad_gb300 import ops
+    n = 4000
+    sites = _tall(w, h, n)
+    near = np.searchsorted(sites[:, 1], np.arange(h)).repeat(w)[:, None] + np.arange(-4, 4)
+    ids = near.clip(0, n - 1).astype(np.uint32)
+    c0, c1 = np.ascontiguousarray(ids[:, :4]), np.ascontiguousarray(ids[:, 4:])
+    img = np.random.default_rng(3).uniform(0, 1, (h, w, 3)).astype(np.float32)
+    dev = lambda a: torch.from_numpy(a.view(np.int32) if a.dtype == np.uint32 else a).cuda()  # noqa: E731
+    bufs = [torch.zeros(n, device="cuda") for _ in range(11)]
+    inv = 1.0 / max(w, h) ** 2
+    ops.compute_gradients_tiled(dev(c0), dev(c1), dev(img), dev(img), torch.ones(h, w, device="cuda"), dev(sites), *bufs,
+                                inv, 0, 0, 0.0, w, h)
+    want = orc.compute_gradients_d(c0, c1, img, sites, w, h)
+    for b, g in zip(bufs, want):
+        assert np.linalg.norm(b.cpu().numpy() - g) <= 1e-3 * np.linalg.norm(g)
+
+
 def test_render_of_a_tall_image(cuda):
     """A render from sites whose flood has more rows of blocks than the grid's y takes: pixels
     between 0.2 and 0.8, the range of the sites' colours."""
