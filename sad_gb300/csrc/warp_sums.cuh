@@ -6,7 +6,7 @@
 // whose 64 candidates name some 10-20 distinct sites) takes one site after the other, the
 // smallest id left first: the lanes that list it compute their terms, a folding butterfly
 // sums them over the group and leaves each lane two of the sums at most, which go to global
-// memory by one reduction per value.  No shared memory, no key table, no barrier.
+// memory by one reduction per value.  No add in shared memory, and one barrier in the block.
 // What is the same for every pixel of a site (softness, scales) is multiplied in after the
 // sum.  Groups of 8 balance the site loop's length, which falls with the group (fewer
 // distinct sites, fewer idle lanes), against the global reductions, which rise: a 1999x1503
@@ -15,10 +15,10 @@
 // head instead of scanning eight ids for the minimum and for each match (some 20 of 150
 // instructions a round): 372 instead of 394 us there from site records; step at 1237x941 with
 // SSIM and removal deltas 325 instead of 328 us.
-// Lists without common sites (a random initial field) would make that loop long: once the
-// first sites turn out to be shared by few lanes, the block collects what is left in a key
-// table in shared memory, whose float adds rarely meet then (added straight to global memory,
-// the terms' arbitrary order would show in more of the sums' last bits).
+// Lists with little in common (a random initial field) would make that loop long: a warp with
+// such a group (kMostMarks) leaves its pixels to a key table of the block in shared memory,
+// whose float adds rarely meet then (added straight to global memory, the terms' arbitrary
+// order would show in more of the sums' last bits).
 #pragma once
 
 #include "accum.cuh"
@@ -28,7 +28,7 @@
 namespace sad {
 
 constexpr int kSumGroup = 8;
-constexpr int kSumSlots = 256;  // keys of the block's table
+constexpr int kSumSlots = 512;  // keys of the block's table
 
 // Pixel of a lane in its warp's 8x4 patch, with every eight lanes a 4x2 patch.
 __device__ __forceinline__ int2 sum_patch_pixel(int lane) {
@@ -142,7 +142,30 @@ __device__ __forceinline__ void sort_candidates(uint32_t (&ids)[kCand], float (&
     }
 }
 
-// What the site loop leaves of a pixel's candidates, for add_by_table.
+// How many of 64 hash values the ids of the lane's group take: 64 (1 - e^(-d/64)) for d distinct
+// ids, give or take two.  Some 27 sites, or rounds of the loop, are its limit, which a field of
+// one site a pixel still keeps: the adjoint at 256x256 with 65,536 sites takes 25 us with a
+// limit of 22 marks, 46 with 19; at 512x512 with 262,144 sites 52 and 72 us; from random lists
+// of 256 sites at 181x181, where the longest loop counts, 41 us, with a limit of 25 marks the
+// same, of 19 marks 39 us.
+constexpr int kMostMarks = 22;
+__device__ __forceinline__ int distinct_marks(const uint32_t (&ids)[kCand]) {
+    uint32_t lo = 0u, hi = 0u;
+#pragma unroll
+    for (int i = 0; i < kCand; ++i) {
+        const uint32_t h = (ids[i] * 2654435761u) >> 26, bit = ids[i] == kEmpty ? 0u : 1u << (h & 31u);
+        lo |= h & 32u ? 0u : bit;
+        hi |= h & 32u ? bit : 0u;
+    }
+#pragma unroll
+    for (int m = kSumGroup / 2; m > 0; m /= 2) {
+        lo |= __shfl_xor_sync(0xffffffffu, lo, m);
+        hi |= __shfl_xor_sync(0xffffffffu, hi, m);
+    }
+    return __popc(lo) + __popc(hi);
+}
+
+// The candidates of a pixel that the site loop leaves, for add_by_table.
 struct LeftCandidates {
     uint32_t ids[kCand];
     float wts[kCand], rem[kCand];
@@ -227,18 +250,14 @@ __device__ __forceinline__ void add_site_gradients(uint32_t (&ids)[kCand], float
     bool by_tau[R];
 #pragma unroll
     for (int k = 0; k < R; ++k) scale[k] = sum_scale(first + k, inv_s2, inv_scale, by_tau[k]);
-    sort_candidates<kRemoval>(ids, wts, rem);
-    // over the first two rounds, at least half a lane's pixel of those that list anything
-    const int enough = __popc(__ballot_sync(full, ids[0] != kEmpty)) / 2;
-    int rounds = 0, members = 0;
-    bool left = true;
+    const bool left = __any_sync(full, distinct_marks(ids) > kMostMarks);  // no loop in this warp
+    if (!left) sort_candidates<kRemoval>(ids, wts, rem);
 #pragma unroll 1
-    while (rounds < 2 || members >= enough) {
+    while (!left) {
         uint32_t id = ids[0];
 #pragma unroll
         for (int m = G / 2; m > 0; m /= 2) id = min(id, __shfl_xor_sync(full, id, m));
-        left = __any_sync(full, id != kEmpty) != 0;
-        if (!left) break;
+        if (!__any_sync(full, id != kEmpty)) break;
         const bool mine = ids[0] == id && id != kEmpty;  // a repeated id comes again
         const float w = wts[0], r = kRemoval ? rem[0] : 0.0f;
         if (mine) {
@@ -246,10 +265,6 @@ __device__ __forceinline__ void add_site_gradients(uint32_t (&ids)[kCand], float
             shift8(wts);
             if constexpr (kRemoval) shift8(rem);
             ids[kCand - 1] = kEmpty;
-        }
-        if (rounds < 2) {
-            members += __popc(__ballot_sync(full, mine));
-            ++rounds;
         }
         float v[NV];
 #pragma unroll
