@@ -221,13 +221,15 @@ __device__ __forceinline__ void candidate_values(const SiteGeom& g, float3 col, 
 // sites takes 181 us, 276 us with a key table and float adds in shared memory; at 1237x941
 // with SSIM and removal deltas 318 instead of 575 us.  Four blocks per SM (64 registers): with
 // three or five the latter takes 322 us.
-template <class Src, bool kRemoval, bool kSSIM>
+template <class Src, bool kRemoval, bool kSSIM, bool kTable>
 __global__ void __launch_bounds__(256, 4)
     fused_gradients_kernel(const __grid_constant__ GradParams prm, Src src) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int2 at = sum_patch_pixel(lane);
-    const int x = blockIdx.x * 32 + (warp & 3) * 8 + at.x;
-    const int y = (blockIdx.z * gridDim.y + blockIdx.y) * 8 + (warp >> 2) * 4 + at.y;
+    constexpr int across = kTable ? 2 : 4;  // warps side by side: 16x16 pixels by table, else 32x8
+    const int by = blockIdx.z * gridDim.y + blockIdx.y;
+    const int x = (blockIdx.x * across + warp % across) * 8 + at.x;
+    const int y = (by * (8 / across) + warp / across) * 4 + at.y;
     const int w = prm.width, h = prm.height;
     const float inv_s2 = prm.inv_scale_sq;
     const float inv_scale = sqrtf(inv_s2);
@@ -270,14 +272,19 @@ __global__ void __launch_bounds__(256, 4)
         src.load(id, g, c);
         if (!(g.l1 >= 1e-8f)) g.l2 = 1.0f / 1e-8f;  // l2 = 1 / max(l1, 1e-8) (gradients.cu:383)
     };
-    add_site_gradients<kRemoval>(
-        ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred, load,
-        [&](uint32_t id, int k, float v) { atomicAdd((k < 10 ? prm.soa[k < 10 ? k : 0] : prm.removal) + id, v); },
-        [&](const LeftCandidates& left) {
-            add_by_table<kRemoval>(left, load, [p = &prm](uint32_t id, int k, float v) {
-                atomicAdd((k < 10 ? p->soa[k < 10 ? k : 0] : p->removal) + id, v);
+    const auto add = [&](uint32_t id, int k, float v) {
+        atomicAdd((k < 10 ? prm.soa[k < 10 ? k : 0] : prm.removal) + id, v);
+    };
+    if constexpr (kTable) {
+        sum_by_table<kRemoval>(ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred, load, add);
+    } else {
+        add_site_gradients<kRemoval>(
+            ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred, load, add, [&](const LeftCandidates& left) {
+                add_by_table<kRemoval>(left, load, [p = &prm](uint32_t id, int k, float v) {
+                    atomicAdd((k < 10 ? p->soa[k < 10 ? k : 0] : p->removal) + id, v);
+                });
             });
-        });
+    }
 }
 
 // Trainer form with the candidate field's registration precomputed (register_tiles_kernel):
@@ -628,11 +635,15 @@ cudaError_t prepare_gradient_kernels() {
 template <class Src>
 static void launch_gradients_float(const GradParams& p, Src src, cudaStream_t st) {
     // rows of blocks past the limit of the grid's y are halved into z: 1,048,560 rows, as with 16 a block
-    const int rows = (p.height + 7) / 8, folds = rows > kMaxGridRows ? 2 : 1;
-    const dim3 grid((p.width + 31) / 32, (rows + folds - 1) / folds, folds);
+    const bool by_table = sums_by_table(kGradientTable, p.site_count, p.width, p.height);
+    const int bw = by_table ? 16 : 32, bh = by_table ? 16 : 8;
+    const int rows = (p.height + bh - 1) / bh, folds = rows > kMaxGridRows ? 2 : 1;
+    const dim3 grid((p.width + bw - 1) / bw, (rows + folds - 1) / folds, folds);
     with_constant(p.compute_removal != 0, [&](auto removal) {
         with_constant(p.ssim_weight > 0.0f, [&](auto ssim) {
-            fused_gradients_kernel<Src, removal, ssim><<<grid, 256, 0, st>>>(p, src);
+            with_constant(by_table, [&](auto table) {
+                fused_gradients_kernel<Src, removal, ssim, table><<<grid, 256, 0, st>>>(p, src);
+            });
         });
     });
     note_launches(1);

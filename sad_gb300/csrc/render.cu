@@ -201,7 +201,7 @@ void launch_clear_candidates(uint32_t* c0, uint32_t* c1, int w, int h, cudaStrea
 // with 16,384 raw ones 50 us with the operator around it, against 875 and 99 us with a key table
 // and float adds in shared memory.  Four blocks per SM (64 registers): a render and its adjoint
 // at 1999x1503 take 372 us, with three 415 us, with five 382 us.
-template <class Src>
+template <class Src, bool kTable>
 __global__ void __launch_bounds__(256, 4) render_backward_kernel(
     const uint4* __restrict__ cand0, const uint4* __restrict__ cand1,
     const float* __restrict__ grad_rgb, float* __restrict__ grad_sites, Src src, float inv_s2,
@@ -283,17 +283,22 @@ __global__ void __launch_bounds__(256, 4) render_backward_kernel(
     const auto add = [=](uint32_t id, int k, float v) {
         atomicAdd(grad_sites + static_cast<size_t>(id) * 10 + k, v);
     };
-    add_site_gradients<false>(ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred, load, add,
-                              [&](const LeftCandidates& left) { add_by_table<false>(left, load, add); });
+    if constexpr (kTable)
+        sum_by_table<false>(ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred, load, add);
+    else
+        add_site_gradients<false>(ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred, load, add,
+                                  [&](const LeftCandidates& left) { add_by_table<false>(left, load, add); });
 }
 
 template <class Src>
 static void launch_render_backward(const uint32_t* c0, const uint32_t* c1, const float* grad_rgb,
                                    float* grad_sites, Src src, float inv_s2, uint32_t n,
                                    int w, int h, int cw, int ch, cudaStream_t st) {
-    render_backward_kernel<Src><<<pixel_grid(w, h), dim3(32, 8), 0, st>>>(
-        reinterpret_cast<const uint4*>(c0), reinterpret_cast<const uint4*>(c1), grad_rgb, grad_sites, src,
-        inv_s2, n, w, h, cw, ch);
+    const auto kernel = sums_by_table(kAdjointTable, n, w, h) ? render_backward_kernel<Src, true>
+                                                          : render_backward_kernel<Src, false>;
+    kernel<<<pixel_grid(w, h), dim3(32, 8), 0, st>>>(reinterpret_cast<const uint4*>(c0),
+                                                     reinterpret_cast<const uint4*>(c1), grad_rgb, grad_sites, src,
+                                                     inv_s2, n, w, h, cw, ch);
     note_launches(1);
 }
 

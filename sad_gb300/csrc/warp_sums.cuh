@@ -18,7 +18,8 @@
 // Lists with little in common (a random initial field) would make that loop long: a warp with
 // such a group (kMostMarks) leaves its pixels to a key table of the block in shared memory,
 // whose float adds rarely meet then (added straight to global memory, the terms' arbitrary
-// order would show in more of the sums' last bits).
+// order would show in more of the sums' last bits).  With few sites on many pixels all sums go
+// that way (TableRule).
 #pragma once
 
 #include "accum.cuh"
@@ -29,6 +30,23 @@ namespace sad {
 
 constexpr int kSumGroup = 8;
 constexpr int kSumSlots = 512;  // keys of the block's table
+
+// Whether all sums go through the table: with few sites on many pixels the groups' reductions
+// queue up at the same addresses in L2 (1999x1503 with 64 sites: the adjoint 2775 us, 759 by
+// table; the gradients with SSIM and removal deltas 3978 and 899 us), and a table holds every
+// site.  The line lies where the two meet on nearest-site fields: at one site per `per_site`
+// pixels on small images and at `most` sites on large ones.  Adjoint by groups and by table: at
+// 256x256 with 64 sites 75 and 45 us, with 100 sites 48 and 46; at 1024x1024 with 300 sites 362 and
+// 317, with 400 sites 271 and 323.  Gradients: at 256x256 with 100 sites 79 and 53 us, with 256
+// sites 46 and 55; at 1024x1024 with 300 sites 441 and 381, with 512 sites 374 and 392.
+struct TableRule {
+    int per_site;
+    uint32_t most;
+};
+constexpr TableRule kAdjointTable = {1000, 300}, kGradientTable = {320, 400};
+inline bool sums_by_table(const TableRule& rule, uint32_t n, int w, int h) {
+    return n <= rule.most && static_cast<double>(w) * h >= static_cast<double>(rule.per_site) * n;
+}
 
 // Pixel of a lane in its warp's 8x4 patch, with every eight lanes a 4x2 patch.
 __device__ __forceinline__ int2 sum_patch_pixel(int lane) {
@@ -173,20 +191,13 @@ struct LeftCandidates {
     float3 dLdp, pred;
 };
 
-// Adds them through a key table of the block (all 256 threads call it).  A call of its own, and
-// with arguments of its own: inlined, its registers cost the site loop 6% (1999x1503: 419
-// instead of 395 us).
+// Adds a block's candidates through its key table (all 256 threads call it; ids: kEmpty where a
+// slot carries none).
 template <bool kRemoval, class Load, class Add>
-__device__ __noinline__ void add_by_table(const LeftCandidates& left, Load load, Add add) {
+__device__ __forceinline__ void sum_by_table(uint32_t (&ids)[kCand], float (&wts)[kCand], float (&rem)[kCand],
+                                             float ux, float uy, float inv_s2, float inv_scale, float3 dLdp,
+                                             float3 pred, Load load, Add add) {
     constexpr int NV = kRemoval ? 11 : 10;
-    uint32_t ids[kCand];
-    float wts[kCand], rem[kCand];
-#pragma unroll
-    for (int i = 0; i < kCand; ++i) {
-        ids[i] = left.ids[i];
-        wts[i] = left.wts[i];
-        if constexpr (kRemoval) rem[i] = left.rem[i];
-    }
     __shared__ TileTable<NV, kSumSlots, AccFloat> table;
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     table.init(tid, 256);
@@ -206,8 +217,7 @@ __device__ __noinline__ void add_by_table(const LeftCandidates& left, Load load,
             float3 col;
             load(ids[0], g, col);
             float o[10], v[NV];
-            candidate_grads(g, col, left.ux, left.uy, left.inv_s2, left.inv_scale, wts[0], left.dLdp, left.pred, false,
-                            o);
+            candidate_grads(g, col, ux, uy, inv_s2, inv_scale, wts[0], dLdp, pred, false, o);
 #pragma unroll
             for (int k = 0; k < 10; ++k) v[k] = o[k];
             if constexpr (kRemoval) v[10] = rem[0];
@@ -231,6 +241,20 @@ __device__ __noinline__ void add_by_table(const LeftCandidates& left, Load load,
     }
 }
 
+// The same for what the site loop leaves: a call of its own, and with arguments of its own:
+// inlined, its registers cost the site loop 6% (1999x1503: 419 instead of 395 us).
+template <bool kRemoval, class Load, class Add>
+__device__ __noinline__ void add_by_table(const LeftCandidates& left, Load load, Add add) {
+    uint32_t ids[kCand];
+    float wts[kCand], rem[kCand];
+#pragma unroll
+    for (int i = 0; i < kCand; ++i) {
+        ids[i] = left.ids[i];
+        wts[i] = left.wts[i];
+        if constexpr (kRemoval) rem[i] = left.rem[i];
+    }
+    sum_by_table<kRemoval>(ids, wts, rem, left.ux, left.uy, left.inv_s2, left.inv_scale, left.dLdp, left.pred, load, add);
+}
 
 // Adds the gradients of a block's pixels (all 256 threads call it; ids: kEmpty where a slot
 // carries none).  load(id, geom, colour) reads a site; add(id, k, value) adds to value k of a
