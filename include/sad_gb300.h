@@ -525,7 +525,10 @@ sad_status_t sad_batch_gradient_ms(sad_batch_t* b, double* ms_per_launch);
 /* ------------------------------------------------------------------------ */
 
 /* Build the candidate field (JFA rounds + VPT passes) for n sites and render it.
- * sites and out_rgb are device pointers; scratch is sad_render_scratch_bytes().
+ * sites and out_rgb are device pointers; scratch is sad_render_scratch_bytes(), 96 bytes a
+ * texel and some 100 a site.  From sad_render_scratch_min_bytes(), 32 bytes a texel less, on
+ * the call is taken too, with the same image: the passes then compute their lists' distances
+ * anew instead of keeping them.
  * replaces: renderVoronoiFromSites, backends/cuda/src/sad_cuda.cu:1678-1858 */
 typedef struct {
     int candidate_passes;   /* --render-cand-passes (16) */
@@ -540,6 +543,7 @@ typedef struct {
 } sad_render_config_t;
 void sad_render_config_default(sad_render_config_t* cfg);
 size_t sad_render_scratch_bytes(uint32_t site_count, int width, int height, int cand_downscale);
+size_t sad_render_scratch_min_bytes(uint32_t site_count, int width, int height, int cand_downscale);
 sad_status_t sad_render_from_sites(const sad_render_config_t* cfg, const float* sites,
                                    uint32_t site_count, int width, int height, float* out_rgb,
                                    void* scratch, size_t scratch_bytes, sad_stream_t stream);

@@ -149,6 +149,7 @@ SIGNATURES = {
     "sad_trainer_fit_host": (st, [vp, vp, vp, vp, i32, C.POINTER(i32), C.POINTER(f32)]),
     "sad_render_config_default": (None, [C.POINTER(RenderConfig)]),
     "sad_render_scratch_bytes": (sz, [u32, i32, i32, i32]),
+    "sad_render_scratch_min_bytes": (sz, [u32, i32, i32, i32]),
     "sad_render_from_sites": (st, [C.POINTER(RenderConfig), vp, u32, i32, i32, vp, vp, sz, vp]),
     "sad_render_from_sites_timed": (st, [C.POINTER(RenderConfig), vp, u32, i32, i32, vp, vp, sz, vp,
                                          C.POINTER(f32), C.POINTER(f32)]),

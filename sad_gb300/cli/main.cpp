@@ -667,7 +667,9 @@ int render(Options& o) {
     const size_t npix = static_cast<size_t>(w) * h;
     DeviceBuf<float> d_sites(ls.sites.size()), d_out(npix * 3);
     check_cuda(cudaMemcpy(d_sites.p, ls.sites.data(), ls.sites.size() * 4, cudaMemcpyHostToDevice), "upload");
-    size_t scratch_bytes = sad_render_scratch_bytes(n, w, h, o.rcfg.cand_downscale);
+    size_t scratch_bytes = sad_render_scratch_bytes(n, w, h, o.rcfg.cand_downscale), free_bytes = 0, total_bytes = 0;
+    check_cuda(cudaMemGetInfo(&free_bytes, &total_bytes), "memory info");
+    if (scratch_bytes > free_bytes) scratch_bytes = sad_render_scratch_min_bytes(n, w, h, o.rcfg.cand_downscale);
     DeviceBuf<unsigned char> d_scratch(scratch_bytes);
     DeviceBuf<uint32_t> d_packed(o.render_packed ? size_t(n) * 4 : 1);
     DeviceBuf<sad_packed_quant_t> d_quant(1);

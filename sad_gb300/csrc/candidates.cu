@@ -426,7 +426,7 @@ __device__ __forceinline__ void vpt_pixel(const VptParams& prm, const Src& src, 
     }
     reinterpret_cast<uint4*>(prm.out0)[p] = make_uint4(bi[0], bi[1], bi[2], bi[3]);
     reinterpret_cast<uint4*>(prm.out1)[p] = make_uint4(bi[4], bi[5], bi[6], bi[7]);
-    if (prm.distances) {
+    if (prm.keep_distances) {
         prm.distances[2 * p] = make_float4(bd[0], bd[1], bd[2], bd[3]);
         prm.distances[2 * p + 1] = make_float4(bd[4], bd[5], bd[6], bd[7]);
     }

@@ -54,15 +54,14 @@ struct Request {
     float* rgb_out = nullptr;
     sad_request_result_t* result = nullptr;
     size_t need = 0;
+    size_t min_need = 0;  // a render's slab where `need` cannot be had (0: no smaller one)
     Clock::time_point submitted;
 };
 
 inline size_t a256(size_t x) { return (x + 255) & ~size_t(255); }
 
-size_t render_need(const sad_render_config_t& c, uint32_t n, int w, int h) {
-    return 256 + a256(size_t(n) * 40) + a256(size_t(w) * h * 12) +
-           sad_render_scratch_bytes(n, w, h, c.cand_downscale);
-}
+// A render's sites and pixels; its scratch follows.
+size_t render_buffers(uint32_t n, int w, int h) { return 256 + a256(size_t(n) * 40) + a256(size_t(w) * h * 12); }
 
 void set_message(sad_request_result_t* r, sad_status_t st) {
     r->status = st;
@@ -128,7 +127,7 @@ sad_status_t run_render(const Request& q, void* mem, cudaStream_t ws) {
     float* rgb = reinterpret_cast<float*>(p);
     size_t npx = size_t(q.w) * q.h;
     p += a256(npx * 12);
-    size_t scratch = sad_render_scratch_bytes(q.n, q.w, q.h, q.rcfg.cand_downscale);
+    const size_t scratch = q.need - render_buffers(q.n, q.w, q.h);
     SAD_TRY(sad::check_cuda(cudaMemcpyAsync(sites, q.sites_in, size_t(q.n) * 40, cudaMemcpyHostToDevice, ws),
                             "executor render: sites upload"));
     SAD_TRY(sad_render_from_sites(&q.rcfg, sites, q.n, q.w, q.h, rgb, p, scratch,
@@ -261,7 +260,17 @@ void worker_main(sad_executor* ex) {
             st = SAD_ERR_INVALID_ARGUMENT;
         }
         if (st == SAD_OK && q.need > 0) {
-            st = sad::check_cuda(cudaMallocAsync(&mem, q.need, ws), "executor: slab allocation");
+            cudaError_t e = cudaMallocAsync(&mem, q.need, ws);
+            if (e == cudaErrorMemoryAllocation && q.min_need > 0 && q.min_need < q.need) {
+                cudaGetLastError();
+                {
+                    std::lock_guard<std::mutex> lock(ex->mu);
+                    ex->in_use -= q.need - q.min_need;
+                }
+                q.need = q.min_need;
+                e = cudaMallocAsync(&mem, q.need, ws);
+            }
+            st = sad::check_cuda(e, "executor: slab allocation");
             if (st == SAD_OK) st = sad::check_cuda(cudaStreamSynchronize(ws), "executor: slab allocation");
         }
         bool keep_slab = false;  // an opened session keeps its slab and its share of the budget
@@ -407,7 +416,11 @@ extern "C" sad_status_t sad_executor_submit_render(sad_executor_t* ex, const sad
     q.h = height;
     q.rgb_out = rgb_host;
     q.result = result;
-    q.need = render_need(*cfg, site_count, width, height);
+    const size_t buffers = render_buffers(site_count, width, height);
+    q.min_need = buffers + sad_render_scratch_min_bytes(site_count, width, height, cfg->cand_downscale);
+    // within a budget the smaller slab: as many renders at a time
+    q.need = ex->budget > 0 ? q.min_need
+                            : buffers + sad_render_scratch_bytes(site_count, width, height, cfg->cand_downscale);
     return enqueue(ex, std::move(q), ticket);
 }
 

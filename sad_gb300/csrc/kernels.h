@@ -77,11 +77,10 @@ struct VptParams {
     const DevState* state;
     uint32_t pass_offset;
     uint32_t pow2, stages;
-    // passes over the same sites (a render): [texels][2] distances of the field's entries,
-    // written by each pass (nullptr: not kept) and read by it when the last pass wrote the
-    // field and them
+    // passes over the same sites (a render): [texels][2] distances of the field's entries, read
+    // where the last pass wrote the field and them, written where the next pass reads them
     float4* distances;
-    bool have_distances;
+    bool have_distances, keep_distances;
 };
 
 // Batched VPT pass: one grid over the 32x8 blocks of every image (host arrays: items[n],

@@ -22,12 +22,12 @@ struct RenderScratch {
     SiteGeom* vgeom;
     uint32_t* c0[2];
     uint32_t* c1[2];
-    float4* distances;  // of the last pass's candidates
     uint32_t* horder;
     uint32_t* hpos;
     uint32_t* hpairs;
     void* sort_temp;
-    size_t total;
+    float4* distances;  // of the last pass's candidates, if there is room
+    size_t total, full;  // bytes without and with the distances
 };
 
 static RenderScratch carve(void* base, uint32_t n, int cw, int ch) {
@@ -48,12 +48,13 @@ static RenderScratch carve(void* base, uint32_t n, int cw, int ch) {
         r.c0[b] = reinterpret_cast<uint32_t*>(take(nc));
         r.c1[b] = reinterpret_cast<uint32_t*>(take(nc));
     }
-    r.distances = reinterpret_cast<float4*>(take(2 * nc));
     r.horder = reinterpret_cast<uint32_t*>(take(static_cast<size_t>(n) * 4));
     r.hpos = reinterpret_cast<uint32_t*>(take(static_cast<size_t>(n) * 4));
     r.hpairs = reinterpret_cast<uint32_t*>(take(static_cast<size_t>(padded) * 8));
     r.sort_temp = take(radix_sort_temp_bytes(padded));
     r.total = off + 256;
+    r.distances = reinterpret_cast<float4*>(take(2 * nc));
+    r.full = off + 256;
     return r;
 }
 
@@ -63,6 +64,13 @@ using namespace sad;
 
 extern "C" size_t sad_render_scratch_bytes(uint32_t site_count, int width, int height,
                                            int cand_downscale) {
+    int ds = std::max(1, cand_downscale);
+    int cw = std::max(1, (width + ds - 1) / ds), ch = std::max(1, (height + ds - 1) / ds);
+    return carve(nullptr, site_count, cw, ch).full;
+}
+
+extern "C" size_t sad_render_scratch_min_bytes(uint32_t site_count, int width, int height,
+                                               int cand_downscale) {
     int ds = std::max(1, cand_downscale);
     int cw = std::max(1, (width + ds - 1) / ds), ch = std::max(1, (height + ds - 1) / ds);
     return carve(nullptr, site_count, cw, ch).total;
@@ -81,7 +89,7 @@ static sad_status_t render_from_sites_impl(const sad_render_config_t* cfg, const
     int cw = std::max(1, (width + ds - 1) / ds), ch = std::max(1, (height + ds - 1) / ds);
     RenderScratch need = carve(nullptr, n, cw, ch);
     SAD_REQUIRE(scratch_bytes >= need.total,
-                "sad_render_from_sites: scratch smaller than sad_render_scratch_bytes()");
+                "sad_render_from_sites: scratch smaller than sad_render_scratch_min_bytes()");
     uintptr_t base = (reinterpret_cast<uintptr_t>(scratch) + 255) & ~uintptr_t(255);
     RenderScratch r = carve(reinterpret_cast<void*>(base), n, cw, ch);
     cudaStream_t st = as_stream(stream);
@@ -144,8 +152,10 @@ static sad_status_t render_from_sites_impl(const sad_render_config_t* cfg, const
         p.height = ch;
         p.state = nullptr;
         p.distances = r.distances;
+        const bool keep = scratch_bytes >= need.full;
         for (int i = 0; i < this_passes; ++i) {
-            p.have_distances = i > 0;  // a round's first pass reads the flood's field
+            p.have_distances = keep && i > 0;  // a round's first pass reads the flood's field
+            p.keep_distances = keep && i + 1 < this_passes;
             p.step = sad_pack_jump_step(jump_pass, cw, ch);
             p.step_high = jump_pass >> 16;
             p.in0 = r.c0[a];

@@ -90,6 +90,14 @@ def test_scratch_queries_are_monotone(sadlib):
     assert sadlib.sad_init_temp_bytes(128000) > 128000 * 4
 
 
+def test_render_scratch_without_distances(sadlib):
+    """The smallest scratch of a render is 32 bytes a texel less."""
+    for w, h, ds in [(256, 256, 1), (301, 199, 1), (301, 199, 2)]:
+        texels = -(-w // ds) * -(-h // ds)
+        saved = sadlib.sad_render_scratch_bytes(1000, w, h, ds) - sadlib.sad_render_scratch_min_bytes(1000, w, h, ds)
+        assert 0 <= saved - 32 * texels < 256
+
+
 def test_default_config_is_the_reference_training_config(sadlib):
     from sad_gb300 import _lib, config
     cfg = config.train_config()

@@ -219,3 +219,52 @@ def test_executor_survives_refused_slabs(cuda):
         ex.wait_all()
         for r in more:
             np.testing.assert_array_equal(r.result(), want)
+
+
+@pytest.mark.parametrize("w,h,passes,rounds", [(64, 48, 16, 1), (130, 77, 5, 2), (96, 96, 1, 1), (33, 40, 0, 1)])
+def test_render_in_the_smallest_scratch(cuda, w, h, passes, rounds):
+    """64 bytes a texel (two fields) and the sites' buffers, without room for the distances that
+    a pass keeps for the next: the same image."""
+    from sad_gb300 import _lib
+    lib = _lib.load()
+    n = 500
+    sites = torch.from_numpy(np.ascontiguousarray(cases.scene(w, h, n, 3)[1])).cuda()
+    cfg = _lib.RenderConfig()
+    lib.sad_render_config_default(C.byref(cfg))
+    cfg.candidate_passes, cfg.jfa_rounds = passes, rounds
+    full = lib.sad_render_scratch_bytes(n, w, h, 1)
+    least = full - (32 * w * h + 255) // 256 * 256
+    images = []
+    for nb in (full, least):
+        scratch = torch.empty(nb, dtype=torch.uint8, device="cuda")
+        out = torch.zeros((h, w, 3), device="cuda")
+        _lib.call("sad_render_from_sites", C.byref(cfg), C.c_void_p(sites.data_ptr()), n, w, h,
+                  C.c_void_p(out.data_ptr()), C.c_void_p(scratch.data_ptr()), nb, None)
+        torch.cuda.synchronize()
+        images.append(out)
+    assert torch.equal(*images)
+    with pytest.raises(_lib.SadError, match="scratch smaller"):
+        _lib.call("sad_render_from_sites", C.byref(cfg), C.c_void_p(sites.data_ptr()), n, w, h,
+                  C.c_void_p(out.data_ptr()), C.c_void_p(scratch.data_ptr()), least - 1, None)
+
+
+def test_renders_within_a_budget_take_the_smallest_slab(cuda):
+    """A budget of one smallest slab: the render stays within it (the default pool's high-water
+    mark), and its image is that of a render with the whole scratch."""
+    from sad_gb300 import _lib
+    from sad_gb300.executor import Executor
+    driver = C.CDLL("libcuda.so.1")
+    pool, used, high = C.c_void_p(), C.c_uint64(0), 8  # CU_MEMPOOL_ATTR_USED_MEM_HIGH
+    assert driver.cuDeviceGetDefaultMemPool(C.byref(pool), torch.cuda.current_device()) == 0
+    assert driver.cuMemPoolSetAttribute(pool, high, C.byref(used)) == 0
+    w, h, n = 512, 384, 2000
+    sites = cases.scene(w, h, n, 4)[1]
+    a256 = lambda x: (x + 255) // 256 * 256  # noqa: E731
+    budget = (256 + a256(40 * n) + a256(12 * w * h) + _lib.fn("sad_render_scratch_bytes")(n, w, h, 1)
+              - a256(32 * w * h))
+    with Executor(workers=2, hbm_budget_bytes=budget) as ex:
+        images = [r.result() for r in [ex.submit_render(sites, w, h) for _ in range(4)]]
+    assert driver.cuMemPoolGetAttribute(pool, high, C.byref(used)) == 0
+    assert 0 < used.value <= budget + (1 << 20)  # the pool's granularity
+    for im in images:
+        np.testing.assert_array_equal(im, solo_render(sites, w, h))
