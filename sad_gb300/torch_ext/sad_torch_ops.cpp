@@ -64,8 +64,14 @@ uint32_t u32(int64_t v) { return static_cast<uint32_t>(v); }
 constexpr int64_t kRecordPixels = 1 << 19;
 bool records_pay(int64_t pixels, int64_t sites) { return pixels >= kRecordPixels && sites <= pixels; }
 
+// Scratch for the records; undefined where there is no memory for them, and the caller takes
+// the kernels that read the sites as they are.
 Tensor scratch_for(const Tensor& like, size_t bytes) {
-    return at::empty({static_cast<int64_t>(bytes)}, like.options().dtype(at::kByte));
+    try {
+        return at::empty({static_cast<int64_t>(bytes)}, like.options().dtype(at::kByte));
+    } catch (const c10::OutOfMemoryError&) {
+        return Tensor();
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -85,8 +91,10 @@ Tensor render_sad_padded(const Tensor& cand0_, const Tensor& cand1_, const Tenso
     c10::cuda::CUDAGuard guard(cand0_.device());
     Tensor cand0 = cand0_.contiguous(), cand1 = cand1_.contiguous(), sites = sites_.contiguous();
     Tensor out = at::empty({height, width, 3}, cand0.options().dtype(at::kFloat));
-    if (records_pay(width * height, sites.size(0))) {
-        Tensor scratch = scratch_for(sites, sad_site_scratch_bytes(u32(sites.size(0))));
+    Tensor scratch;
+    if (records_pay(width * height, sites.size(0)))
+        scratch = scratch_for(sites, sad_site_scratch_bytes(u32(sites.size(0))));
+    if (scratch.defined()) {
         ok(sad_render_in(ptr<uint32_t>(cand0), ptr<uint32_t>(cand1), ptr(out), ptr(sites),
                          static_cast<float>(inv_scale_sq), u32(sites.size(0)), static_cast<int>(width),
                          static_cast<int>(height), static_cast<int>(cand_width), static_cast<int>(cand_height),
@@ -138,6 +146,17 @@ std::tuple<Tensor, Tensor> vpt_pass(const Tensor& cand0_, const Tensor& cand1_, 
     Tensor cand0 = cand0_.contiguous(), cand1 = cand1_.contiguous(), sites = sites_.contiguous();
     Tensor out0 = at::empty_like(cand0), out1 = at::empty_like(cand1);
     Tensor scratch = scratch_for(sites, sad_update_candidates_scratch_bytes(u32(sites.size(0))));
+    if (!scratch.defined()) {  // half as much
+        Tensor packed = at::empty({sites.size(0), 8}, sites.options().dtype(at::kHalf));
+        ok(sad_pack_candidate_sites(ptr(sites), ptr<uint16_t>(packed), u32(sites.size(0)), stream_of(cand0)));
+        ok(sad_update_candidates(ptr<uint32_t>(cand0), ptr<uint32_t>(cand1), ptr<uint32_t>(out0), ptr<uint32_t>(out1),
+                                 ptr<uint16_t>(packed), u32(sites.size(0)), u32(jump << 16),
+                                 static_cast<float>(inv_scale_sq), 0u, static_cast<float>(radius_scale),
+                                 u32(radius_probes), u32(inject_count), nullptr, nullptr, 0u, 0u, 1,
+                                 static_cast<int>(width), static_cast<int>(height), static_cast<int>(width),
+                                 static_cast<int>(height), stream_of(cand0)));
+        return {out0, out1};
+    }
     ok(sad_update_candidates_in(ptr<uint32_t>(cand0), ptr<uint32_t>(cand1), ptr<uint32_t>(out0), ptr<uint32_t>(out1),
                                 nullptr, ptr(sites), u32(sites.size(0)), u32(jump << 16),
                                 static_cast<float>(inv_scale_sq), 0u, static_cast<float>(radius_scale),
@@ -169,8 +188,10 @@ Tensor render_sad_backward(const Tensor& cand0_, const Tensor& cand1_, const Ten
     Tensor grad_sites = clears ? at::empty({sites.size(0), 10}, sites.options())
                                : at::zeros({sites.size(0), 10}, sites.options());
     if (clears) ok(sad_clear_buffer(ptr(grad_sites), u32(grad_sites.numel()), stream_of(cand0)));
-    if (records_pay(width * height, sites.size(0))) {
-        Tensor scratch = scratch_for(sites, sad_site_scratch_bytes(u32(sites.size(0))));
+    Tensor scratch;
+    if (records_pay(width * height, sites.size(0)))
+        scratch = scratch_for(sites, sad_site_scratch_bytes(u32(sites.size(0))));
+    if (scratch.defined()) {
         ok(sad_render_backward_in(ptr<uint32_t>(cand0), ptr<uint32_t>(cand1), ptr(grad_output), ptr(grad_sites),
                                   ptr(sites), static_cast<float>(inv_scale_sq), u32(sites.size(0)),
                                   static_cast<int>(width), static_cast<int>(height), static_cast<int>(width),
@@ -244,9 +265,11 @@ Tensor update_candidates_compact(const Tensor& cand0_in_, const Tensor& cand1_in
         hpp = ptr<uint32_t>(hp);
     }
     // decoding each site once costs a launch: on fields it does not pay for, the pass decodes
+    Tensor scratch;
     if (cand_width * cand_height >= kRecordTexels && site_count <= cand_width * cand_height &&
-        site_count <= packed_sites.size(0)) {
-        Tensor scratch = scratch_for(packed_sites, sad_update_candidates_scratch_bytes(u32(site_count)));
+        site_count <= packed_sites.size(0))
+        scratch = scratch_for(packed_sites, sad_update_candidates_scratch_bytes(u32(site_count)));
+    if (scratch.defined()) {
         ok(sad_update_candidates_in(
             ptr<uint32_t>(cand0_in), ptr<uint32_t>(cand1_in), ptr<uint32_t>(cand0_out), ptr<uint32_t>(cand1_out),
             ptr<uint16_t>(packed_sites), nullptr, u32(site_count), u32(step), static_cast<float>(inv_scale_sq),
@@ -352,8 +375,10 @@ Tensor compute_gradients_tiled(const Tensor& cand0_, const Tensor& cand1_, const
     Tensor cand0 = cand0_.contiguous(), cand1 = cand1_.contiguous(), target = target_.contiguous();
     Tensor rendered = rendered_.contiguous(), mask = mask_.contiguous(), sites = sites_.contiguous();
     if (site_count <= 0) site_count = sites.size(0);
-    if (site_count <= sites.size(0) && records_pay(target.size(0) * target.size(1), site_count)) {
-        Tensor scratch = scratch_for(sites, sad_site_scratch_bytes(u32(site_count)));
+    Tensor scratch;
+    if (site_count <= sites.size(0) && records_pay(target.size(0) * target.size(1), site_count))
+        scratch = scratch_for(sites, sad_site_scratch_bytes(u32(site_count)));
+    if (scratch.defined()) {
         ok(sad_compute_gradients_tiled_in(
             ptr<uint32_t>(cand0), ptr<uint32_t>(cand1), ptr(target), ptr(rendered), ptr(mask), ptr(grad_pos_x),
             ptr(grad_pos_y), ptr(grad_log_tau), ptr(grad_radius), ptr(grad_color_r), ptr(grad_color_g),

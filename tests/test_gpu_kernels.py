@@ -315,6 +315,58 @@ def test_operators_with_site_records(ops, w, h, n):
         assert (a - b).double().norm() <= 1e-5 * b.double().norm()
 
 
+def test_operators_without_memory_for_site_records(ops):
+    """Where the records' scratch cannot be had, the operators take the kernels that read the
+    sites as they are: the same lists and image, and the same float sums up to their order."""
+    w = h = 1024
+    n = 1000000
+    rng = np.random.default_rng(11)
+    sites = tf(cases.scene(w, h, 4096, 3)[1][rng.integers(0, 4096, n)])
+    sites[:, :2] = torch.rand(n, 2, device="cuda") * w
+    sites[::13, 0] = -1.0
+    c0, c1 = [torch.randint(0, n, (w * h, 4), dtype=torch.int32, device="cuda") for _ in range(2)]
+    inv, packed = 1.0 / w ** 2, torch.empty(n, 8, dtype=torch.float16, device="cuda")
+    ops.pack_candidate_sites(sites, packed, n)
+    target, gout = torch.rand(h, w, 3, device="cuda"), torch.randn(h, w, 3, device="cuda")
+    mask, none = torch.ones(h, w, device="cuda"), torch.empty(0, dtype=torch.int32, device="cuda")
+    lists, grads = [torch.empty_like(c) for c in (c0, c1)], _grad_buffers(n)
+
+    def update():
+        ops.update_candidates_compact(c0, c1, *lists, packed, none, none, inv, n, 3 << 16, 0, 1.0, 0, 4, 0, 0, 1, w, h,
+                                      w, h)
+        return lists
+
+    def gradients():
+        for g in grads:
+            g.zero_()
+        ops.compute_gradients_tiled(c0, c1, target, target, mask, sites, *grads, inv, n, 0, 0.0, w, h)
+        return grads[:10]
+
+    mb = 1 << 20
+    # call, MiB that its results and the smaller scratch take, exact
+    calls = [(lambda: [ops.render_sad(c0, c1, sites, inv, w, h)], 12, True), (update, 0, True), (gradients, 0, False),
+             (lambda: ops.render_sad_backward(c0, c1, sites, gout, inv, w, h).unbind(1), 40, False),
+             (lambda: ops.vpt_pass(c0, c1, sites, inv, w, h, 3, 0, 1.0, 4, 0), 32 + 16, True)]
+    total = torch.cuda.get_device_properties(0).total_memory
+    for call, results, exact in calls:
+        want = [x.clone() for x in call()]
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (results + 10) * mb) / total)
+        try:
+            with pytest.raises(torch.OutOfMemoryError):
+                torch.empty((results + 30) * mb, dtype=torch.uint8, device="cuda")
+            got = call()
+            torch.cuda.synchronize()
+        finally:
+            torch.cuda.set_per_process_memory_fraction(1.0)
+        for a, b in zip(got, want):
+            if exact:
+                assert torch.equal(a, b)
+            else:
+                assert (a - b).double().norm() <= 1e-5 * b.double().norm()
+
+
 # ---------------------------------------------------------------------------
 # training kernels
 # ---------------------------------------------------------------------------
