@@ -52,6 +52,25 @@ def test_batch_matches_single_fits_bitwise(cuda, graphs):
         assert (want_sites[:, 0] >= 0).sum() < CFG["n_sites"]  # the prune events ran
 
 
+@pytest.mark.parametrize("n", [4096, 4097])
+def test_batch_matches_either_form_of_the_per_site_work(cuda, n):
+    """A fit alone does the per-site work of an iteration in one launch up to 4,096 sites and in
+    several above; the batch's kernels give the bits of both."""
+    from sad_gb300.batch import Batch
+    cfg = dict(CFG, n_sites=n, max_sites=n, iterations=100)
+    sizes = [(130, 77), (96, 96)]
+    imgs = [synthetic_image(w, h, seed=30 + i) for i, (w, h) in enumerate(sizes)]
+    with Batch(sizes, use_graphs=1, **cfg) as b:
+        for i, img in enumerate(imgs):
+            b.set_target(i, img)
+        b.init()
+        b.run()
+        b.synchronize()
+        got = [b.sites(i, active_only=False) for i in range(len(imgs))]
+    for img, sites in zip(imgs, got):
+        np.testing.assert_array_equal(sites.view(np.uint32), _solo(img, use_graphs=1, **cfg)[0].view(np.uint32))
+
+
 @pytest.mark.parametrize("end", [75, 100])
 def test_fit_that_leaves_the_batch(cuda, end):
     """One image of the batch has a site on most pixels, so the batch marks crowded tiles for

@@ -605,6 +605,36 @@ def test_trainer_gradients_match_oracle(ops, orc, w, h, n, field, removal, maske
         assert not fix[:, 10:].any()
 
 
+@pytest.mark.parametrize("crowded", ["none", "some"])
+@pytest.mark.parametrize("removal", [False, True])
+def test_trainer_gradients_of_full_tables(cuda, orc, crowded, removal):
+    """Tiles that name more sites than a table holds (256) without being crowded: their first two
+    candidates name few, the other six many, so the keys past the table's end add to global
+    memory; and, among them, tiles whose first two candidates already name too many, which use
+    no table.  Soft sites, so that random lists stay well conditioned in FP32."""
+    w, h, n = 80, 48, 3000
+    img, sites = cases.scene(w, h, n, 70)
+    sites[:, 2] = 1.0
+    sites[::9, 0] = -1
+    c0, c1 = cases.random_field(w, h, n, 71, empty_frac=0.0, dup_frac=0.0, invalid_frac=0.0)
+    tile = (np.arange(w * h) % w) // 16 + (np.arange(w * h) // w) // 16 * (w // 16)
+    few = np.ones(w * h, bool) if crowded == "none" else tile % 3 != 0
+    c0[few, :2] = c0[few, :2] % 100 + (tile[few] * 150)[:, None].astype(np.uint32)
+    for t in range(tile.max() + 1):
+        near = np.unique(c0[tile == t, :2]).size
+        assert (near <= 256) == (crowded == "none" or t % 3 != 0)
+        assert np.unique(np.concatenate([c0[tile == t].ravel(), c1[tile == t].ravel()])).size > 512
+    mask, rendered = np.ones((h, w), np.float32), orc.render(c0, c1, sites, w, h)
+    fix, scale = _fixed_gradients(w, h, n, c0, c1, img, rendered, mask, sites, removal, 0.0)
+    again, _ = _fixed_gradients(w, h, n, c0, c1, img, rendered, mask, sites, removal, 0.0)
+    np.testing.assert_array_equal(fix, again)
+    g, a, rem = orc.compute_gradients(c0, c1, img, sites, w, h, rendered=rendered, removal=removal)
+    assert_grads_close(fix[:, :10].T / 2.0 ** 24, g, a, want64=orc.compute_gradients_d(c0, c1, img, sites, w, h))
+    if removal:
+        r = fix[:, 10] / 2.0 ** 24 / scale + fix[:, 11] * 1.0e6
+        assert np.all(np.abs(r - rem) <= 1e-3 * np.maximum(np.abs(rem), 1.0) + 1e-4)
+
+
 @pytest.mark.parametrize("target", [-5.0e11, 4.0e11])
 def test_trainer_gradients_of_large_terms(cuda, orc, target):
     """Terms from 2^27, where a split in two 32-bit words ends, to 2^38, which the 64-bit sums

@@ -44,6 +44,28 @@ def test_trainer_graph_and_eager_agree(cuda):
     np.testing.assert_array_equal(res[1][3], res[0][3])
 
 
+def test_densify_past_the_one_launch_size(cuda):
+    """A fit whose densify steps take it from 3,600 sites past 4,096, where the per-site work goes
+    from one launch to several: graph replays and eager launches agree bit for bit."""
+    from sad_gb300.trainer import Trainer
+    img = cases.scene(120, 100, 6)[0]
+    out = []
+    for graphs in (1, 0):
+        cfg = small_cfg(n_sites=3600, max_sites=5000, iterations=90, densify_start=10, densify_freq=15, densify_end=60,
+                        densify=1, densify_percentile=0.08, prune_start=65, prune_end=85, use_graphs=graphs)
+        with Trainer(120, 100, cfg) as tr:
+            tr.set_target(img)
+            tr.init()
+            first = tr.psnr()
+            tr.run(20)
+            assert tr.info().site_buffer < 4096
+            tr.run()
+            assert tr.info().site_buffer > 4096
+            assert tr.psnr() > first + 3.0
+            out.append(tr.sites(active_only=False))
+    np.testing.assert_array_equal(out[0].view(np.uint32), out[1].view(np.uint32))
+
+
 def test_trainer_fit_is_reproducible(cuda):
     from sad_gb300.trainer import Trainer
     img = cases.scene(96, 96, 5)[0]
