@@ -225,6 +225,7 @@ template <class Src, bool kRemoval, bool kSSIM, bool kTable>
 __global__ void __launch_bounds__(256, 4)
     fused_gradients_kernel(const __grid_constant__ GradParams prm, Src src) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if constexpr (!kTable) begin_sums(threadIdx.x);
     const int2 at = sum_patch_pixel(lane);
     constexpr int across = kTable ? 2 : 4;  // warps side by side: 16x16 pixels by table, else 32x8
     const int by = blockIdx.z * gridDim.y + blockIdx.y;
@@ -279,8 +280,8 @@ __global__ void __launch_bounds__(256, 4)
         sum_by_table<kRemoval>(ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred, load, add);
     } else {
         add_site_gradients<kRemoval>(
-            ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred, load, add, [&](const LeftCandidates& left) {
-                add_by_table<kRemoval>(left, load, [p = &prm](uint32_t id, int k, float v) {
+            ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred, load, add, [&](const PixelCandidates& from) {
+                add_by_table<kRemoval>(from, load, [p = &prm](uint32_t id, int k, float v) {
                     atomicAdd((k < 10 ? p->soa[k < 10 ? k : 0] : p->removal) + id, v);
                 });
             });

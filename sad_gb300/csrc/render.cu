@@ -207,6 +207,7 @@ __global__ void __launch_bounds__(256, 4) render_backward_kernel(
     const float* __restrict__ grad_rgb, float* __restrict__ grad_sites, Src src, float inv_s2,
     uint32_t n, int w, int h, int cw, int ch) {
     const int lane = threadIdx.x, warp = threadIdx.y;
+    if constexpr (!kTable) begin_sums(warp * 32 + lane);
     const int2 at = sum_patch_pixel(lane);
     const int x = blockIdx.x * 32 + (warp & 3) * 8 + at.x;
     const int y = blockIdx.y * 8 + (warp >> 2) * 4 + at.y;
@@ -287,7 +288,7 @@ __global__ void __launch_bounds__(256, 4) render_backward_kernel(
         sum_by_table<false>(ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred, load, add);
     else
         add_site_gradients<false>(ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred, load, add,
-                                  [&](const LeftCandidates& left) { add_by_table<false>(left, load, add); });
+                                  [&](const PixelCandidates& from) { add_by_table<false>(from, load, add); });
 }
 
 template <class Src>

@@ -15,11 +15,10 @@
 // head instead of scanning eight ids for the minimum and for each match (some 20 of 150
 // instructions a round): 372 instead of 394 us there from site records; step at 1237x941 with
 // SSIM and removal deltas 325 instead of 328 us.
-// Lists with little in common (a random initial field) would make that loop long: a warp with
-// such a group (kMostMarks) leaves its pixels to a key table of the block in shared memory,
-// whose float adds rarely meet then (added straight to global memory, the terms' arbitrary
-// order would show in more of the sums' last bits).  With few sites on many pixels all sums go
-// that way (TableRule).
+// Lists with little in common (a random initial field) would make that loop long: a block with
+// such a group (kMostMarks) takes a key table in shared memory instead, whose float adds rarely
+// meet then (added straight to global memory, the terms' arbitrary order would show in more of
+// the sums' last bits).  With few sites on many pixels all sums go that way (TableRule).
 #pragma once
 
 #include "accum.cuh"
@@ -183,8 +182,20 @@ __device__ __forceinline__ int distinct_marks(const uint32_t (&ids)[kCand]) {
     return __popc(lo) + __popc(hi);
 }
 
-// The candidates of a pixel that the site loop leaves, for add_by_table.
-struct LeftCandidates {
+// Whether a warp of the block has left its pixels to the table: the others then leave the site
+// loop, where they would keep it waiting.  begin_sums() before the first loads (a barrier later,
+// where the warps have drifted apart, cost the adjoint at 1999x1503 4%).
+__device__ __forceinline__ volatile int* block_takes_table() {
+    __shared__ int s_takes_table;
+    return &s_takes_table;
+}
+__device__ __forceinline__ void begin_sums(int tid) {
+    if (tid == 0) *block_takes_table() = 0;
+    __syncthreads();
+}
+
+// A pixel's candidates, for add_by_table.
+struct PixelCandidates {
     uint32_t ids[kCand];
     float wts[kCand], rem[kCand];
     float ux, uy, inv_s2, inv_scale;
@@ -241,24 +252,24 @@ __device__ __forceinline__ void sum_by_table(uint32_t (&ids)[kCand], float (&wts
     }
 }
 
-// The same for what the site loop leaves: a call of its own, and with arguments of its own:
-// inlined, its registers cost the site loop 6% (1999x1503: 419 instead of 395 us).
+// The same as a call of its own, and with arguments of its own: inlined beside the site loop, its
+// registers cost the loop 6% (1999x1503: 419 instead of 395 us).
 template <bool kRemoval, class Load, class Add>
-__device__ __noinline__ void add_by_table(const LeftCandidates& left, Load load, Add add) {
+__device__ __noinline__ void add_by_table(const PixelCandidates& from, Load load, Add add) {
     uint32_t ids[kCand];
     float wts[kCand], rem[kCand];
 #pragma unroll
     for (int i = 0; i < kCand; ++i) {
-        ids[i] = left.ids[i];
-        wts[i] = left.wts[i];
-        if constexpr (kRemoval) rem[i] = left.rem[i];
+        ids[i] = from.ids[i];
+        wts[i] = from.wts[i];
+        if constexpr (kRemoval) rem[i] = from.rem[i];
     }
-    sum_by_table<kRemoval>(ids, wts, rem, left.ux, left.uy, left.inv_s2, left.inv_scale, left.dLdp, left.pred, load, add);
+    sum_by_table<kRemoval>(ids, wts, rem, from.ux, from.uy, from.inv_s2, from.inv_scale, from.dLdp, from.pred, load, add);
 }
 
 // Adds the gradients of a block's pixels (all 256 threads call it; ids: kEmpty where a slot
 // carries none).  load(id, geom, colour) reads a site; add(id, k, value) adds to value k of a
-// site: its ten parameters and, with kRemoval, rem[] as value 10; by_table(left) calls
+// site: its ten parameters and, with kRemoval, rem[] as value 10; by_table(from) calls
 // add_by_table.
 template <bool kRemoval, class Load, class Add, class Table>
 __device__ __forceinline__ void add_site_gradients(uint32_t (&ids)[kCand], float (&wts)[kCand],
@@ -274,14 +285,16 @@ __device__ __forceinline__ void add_site_gradients(uint32_t (&ids)[kCand], float
     bool by_tau[R];
 #pragma unroll
     for (int k = 0; k < R; ++k) scale[k] = sum_scale(first + k, inv_s2, inv_scale, by_tau[k]);
-    const bool left = __any_sync(full, distinct_marks(ids) > kMostMarks);  // no loop in this warp
-    if (!left) sort_candidates<kRemoval>(ids, wts, rem);
+    bool left = __any_sync(full, distinct_marks(ids) > kMostMarks);
+    if (left) *block_takes_table() = 1;  // no loop in this warp, and soon none in the others
+    else sort_candidates<kRemoval>(ids, wts, rem);
 #pragma unroll 1
     while (!left) {
+        const int stop = *block_takes_table();
         uint32_t id = ids[0];
 #pragma unroll
         for (int m = G / 2; m > 0; m /= 2) id = min(id, __shfl_xor_sync(full, id, m));
-        if (!__any_sync(full, id != kEmpty)) break;
+        if (!__any_sync(full, id != kEmpty && stop == 0)) break;
         const bool mine = ids[0] == id && id != kEmpty;  // a repeated id comes again
         const float w = wts[0], r = kRemoval ? rem[0] : 0.0f;
         if (mine) {
@@ -310,8 +323,8 @@ __device__ __forceinline__ void add_site_gradients(uint32_t (&ids)[kCand], float
         for (int k = 0; k < R; ++k)
             if (k < count && id != kEmpty) add(id, first + k, s[k] * (scale[k] * (by_tau[k] ? tau : 1.0f)));
     }
-    if (!__syncthreads_or(left)) return;
-    LeftCandidates rest;
+    if (!__syncthreads_or(left || ids[0] != kEmpty)) return;
+    PixelCandidates rest;
 #pragma unroll
     for (int i = 0; i < kCand; ++i) {
         rest.ids[i] = ids[i];

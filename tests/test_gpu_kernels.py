@@ -484,6 +484,28 @@ def test_lists_with_little_in_common_leave_the_loop(ops):
     assert random < 3 * near
 
 
+def test_lists_with_little_in_common_in_a_last_row(ops):
+    """Random lists on 184x181 pixels, whose last row gives each warp groups of four pixels, take
+    the time of 184x184 (1.4 times it where those warps stay in the site loop and the rest of the
+    block waits for them at the table)."""
+    import ctypes as C
+    from sad_gb300 import _lib
+    us = []
+    for w, h in ((184, 181), (184, 184)):
+        c0, c1 = [torch.randint(0, 256, (w * h, 4), dtype=torch.int32, device="cuda",
+                                generator=torch.Generator("cuda").manual_seed(i)) for i in range(2)]
+        sites = tf(cases.scene(w, h, 256, 3)[1])
+        gout, grad = torch.ones(h, w, 3, device="cuda"), torch.zeros_like(sites)
+        ptrs = [C.c_void_p(t.data_ptr()) for t in (c0, c1, gout, grad, sites)]
+        stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+        def calls():
+            for _ in range(30):
+                _lib.call("sad_render_backward", *ptrs, 1.0 / w ** 2, 256, w, h, w, h, stream)
+        us.append(_us(calls))
+    assert us[0] < 1.25 * us[1]
+
+
 def test_few_sites_do_not_serialise(ops):
     """Sums of eight sites on a megapixel: 2.5-3.5 times the time of 4,096 sites' by table, 18-28
     times it by one global reduction for each group of eight lanes."""
