@@ -277,11 +277,11 @@ __global__ void __launch_bounds__(256, 4)
         atomicAdd((k < 10 ? prm.soa[k < 10 ? k : 0] : prm.removal) + id, v);
     };
     if constexpr (kTable) {
-        sum_by_table<kRemoval>(ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred, load, add);
+        sum_by_table<kRemoval, true>(ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred, load, add);
     } else {
         add_site_gradients<kRemoval>(
             ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred, load, add, [&](const PixelCandidates& from) {
-                add_by_table<kRemoval>(from, load, [p = &prm](uint32_t id, int k, float v) {
+                add_by_table<kRemoval, true>(from, load, [p = &prm](uint32_t id, int k, float v) {
                     atomicAdd((k < 10 ? p->soa[k < 10 ? k : 0] : p->removal) + id, v);
                 });
             });

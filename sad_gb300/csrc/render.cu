@@ -285,10 +285,10 @@ __global__ void __launch_bounds__(256, 4) render_backward_kernel(
         atomicAdd(grad_sites + static_cast<size_t>(id) * 10 + k, v);
     };
     if constexpr (kTable)
-        sum_by_table<false>(ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred, load, add);
+        sum_by_table<false, false>(ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred, load, add);
     else
         add_site_gradients<false>(ids, wts, rem, ux, uy, inv_s2, inv_scale, dLdp, pred, load, add,
-                                  [&](const PixelCandidates& from) { add_by_table<false>(from, load, add); });
+                                  [&](const PixelCandidates& from) { add_by_table<false, false>(from, load, add); });
 }
 
 template <class Src>

@@ -203,8 +203,9 @@ struct PixelCandidates {
 };
 
 // Adds a block's candidates through its key table (all 256 threads call it; ids: kEmpty where a
-// slot carries none).
-template <bool kRemoval, class Load, class Add>
+// slot carries none).  kArrays: add() goes to an array per value, where neighbouring lanes take
+// neighbouring sites at the end, instead of neighbouring values of a site's row.
+template <bool kRemoval, bool kArrays, class Load, class Add>
 __device__ __forceinline__ void sum_by_table(uint32_t (&ids)[kCand], float (&wts)[kCand], float (&rem)[kCand],
                                              float ux, float uy, float inv_s2, float inv_scale, float3 dLdp,
                                              float3 pred, Load load, Add add) {
@@ -246,15 +247,22 @@ __device__ __forceinline__ void sum_by_table(uint32_t (&ids)[kCand], float (&wts
     }
     __syncthreads();
     const int used = table.size();
-    for (int q = tid; q < used * NV; q += 256) {
-        const int d = q / NV, k = q - d * NV;
-        add(table.key_at(d), k, table.value(k, d));
+    if constexpr (kArrays) {
+        for (int d = tid; d < used; d += 256) {
+#pragma unroll
+            for (int k = 0; k < NV; ++k) add(table.key_at(d), k, table.value(k, d));
+        }
+    } else {
+        for (int q = tid; q < used * NV; q += 256) {
+            const int d = q / NV, k = q - d * NV;
+            add(table.key_at(d), k, table.value(k, d));
+        }
     }
 }
 
 // The same as a call of its own, and with arguments of its own: inlined beside the site loop, its
 // registers cost the loop 6% (1999x1503: 419 instead of 395 us).
-template <bool kRemoval, class Load, class Add>
+template <bool kRemoval, bool kArrays, class Load, class Add>
 __device__ __noinline__ void add_by_table(const PixelCandidates& from, Load load, Add add) {
     uint32_t ids[kCand];
     float wts[kCand], rem[kCand];
@@ -264,7 +272,8 @@ __device__ __noinline__ void add_by_table(const PixelCandidates& from, Load load
         wts[i] = from.wts[i];
         if constexpr (kRemoval) rem[i] = from.rem[i];
     }
-    sum_by_table<kRemoval>(ids, wts, rem, from.ux, from.uy, from.inv_s2, from.inv_scale, from.dLdp, from.pred, load, add);
+    sum_by_table<kRemoval, kArrays>(ids, wts, rem, from.ux, from.uy, from.inv_s2, from.inv_scale, from.dLdp, from.pred,
+                                    load, add);
 }
 
 // Adds the gradients of a block's pixels (all 256 threads call it; ids: kEmpty where a slot
