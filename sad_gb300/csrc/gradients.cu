@@ -635,10 +635,11 @@ cudaError_t prepare_gradient_kernels() {
 
 template <class Src>
 static void launch_gradients_float(const GradParams& p, Src src, cudaStream_t st) {
-    // rows of blocks past the limit of the grid's y are halved into z: 1,048,560 rows, as with 16 a block
     const bool by_table = sums_by_table(kGradientTable, p.site_count, p.width, p.height);
     const int bw = by_table ? 16 : 32, bh = by_table ? 16 : 8;
-    const int rows = (p.height + bh - 1) / bh, folds = rows > kMaxGridRows ? 2 : 1;
+    // rows of 8-pixel blocks past the limit of the grid's y are halved into z: images of up to
+    // 1,048,560 rows either way
+    const int rows = (p.height + bh - 1) / bh, folds = !by_table && rows > kMaxGridRows ? 2 : 1;
     const dim3 grid((p.width + bw - 1) / bw, (rows + folds - 1) / folds, folds);
     with_constant(p.compute_removal != 0, [&](auto removal) {
         with_constant(p.ssim_weight > 0.0f, [&](auto ssim) {

@@ -114,6 +114,17 @@ def test_gradients_of_tall_images(cuda, orc, w, h):
         assert np.linalg.norm(b.cpu().numpy() - g) <= 1e-3 * np.linalg.norm(g)
 
 
+@pytest.mark.parametrize("n", [8, 4000])  # sums by table, and by groups of lanes
+def test_gradients_of_too_tall_an_image_are_refused(cuda, n):
+    from sad_gb300 import ops
+    w, h = 1, 1048561
+    c = torch.zeros(w * h, 4, dtype=torch.int32, device="cuda")
+    img, bufs = torch.zeros(h, w, 3, device="cuda"), [torch.zeros(n, device="cuda") for _ in range(11)]
+    with pytest.raises(RuntimeError, match="invalid configuration|invalid argument"):
+        ops.compute_gradients_tiled(c, c, img, img, torch.ones(h, w, device="cuda"),
+                                    torch.from_numpy(_tall(w, h, n)).cuda(), *bufs, 1.0 / h ** 2, 0, 0, 0.0, w, h)
+
+
 def test_render_of_a_tall_image(cuda):
     """A render from sites whose flood has more rows of blocks than the grid's y takes: pixels
     between 0.2 and 0.8, the range of the sites' colours."""
