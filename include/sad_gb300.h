@@ -528,7 +528,7 @@ sad_status_t sad_batch_gradient_ms(sad_batch_t* b, double* ms_per_launch);
  * sites and out_rgb are device pointers; scratch is sad_render_scratch_bytes(), 96 bytes a
  * texel and some 100 a site.  From sad_render_scratch_min_bytes(), 32 bytes a texel less, on
  * the call is taken too, with the same image: the passes then compute their lists' distances
- * anew instead of keeping them.
+ * anew instead of keeping them (4096x4096 with 131,072 sites: 33.1 instead of 30.6 ms).
  * replaces: renderVoronoiFromSites, backends/cuda/src/sad_cuda.cu:1678-1858 */
 typedef struct {
     int candidate_passes;   /* --render-cand-passes (16) */

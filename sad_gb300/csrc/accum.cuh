@@ -8,17 +8,18 @@
 // address and the atomics serialise.
 //
 // Here a tile table is filled in two steps:
-//   1. registration: for each candidate slot, __match_any_sync groups the warp's lanes by
-//      site; the group's lowest lane inserts the key (CAS probe) and broadcasts the table
-//      slot, so each key costs one CAS per warp;
-//   2. accumulation: every lane adds its values to the registered slot directly, visiting
+//   1. registration: a key whose first hash slot holds it is found by a plain read; a warp that
+//      misses one groups its lanes by site (__match_any_sync), the group's lowest lane inserts
+//      the key (CAS probe) and broadcasts its table index, so each key costs one CAS per warp;
+//   2. accumulation: every lane adds its values to the registered entry directly, visiting
 //      its 8 candidates in a lane-rotated order so lanes with identical lists hit
-//      different slots at the same instruction.
-// Values are accumulated either as float (API calls, which add into caller buffers like
-// the reference) or as fixed point (the trainer): integer addition is associative, so
-// per-site sums -- and with them whole fits -- are bitwise reproducible.  Keys that do not
-// fit within kMaxProbe probes go to global memory through the caller's fallback, which
-// adds the same integers.
+//      different entries at the same instruction.
+// The trainer's tables hold fixed point: integer addition is associative, so per-site sums --
+// and with them whole fits -- are bitwise reproducible.  Its registration runs once per field
+// refresh (the gradient kernel reads indices), and keys that do not fit in a table, or tiles
+// that have none (kTileCrowded), add the same integers to global memory.  Float tables serve
+// the site statistics of the API and what warp_sums.cuh leaves to them; a key that does not
+// fit within kMaxProbe probes goes to global memory through the caller's fallback.
 #pragma once
 
 #include "common.cuh"

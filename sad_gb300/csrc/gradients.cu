@@ -216,11 +216,12 @@ __device__ __forceinline__ void candidate_values(const SiteGeom& g, float3 col, 
 }
 
 // The API form, adding into the caller's float arrays: 32x8 pixels per block, an 8x4 patch per
-// warp, which sums its sites' gradients by itself (warp_sums.cuh).  Bound by issue.  A torch
-// step (render, gradients, tau diffusion, Adam, candidate refresh) at 768x512 with 24,576
-// sites takes 181 us, 276 us with a key table and float adds in shared memory; at 1237x941
-// with SSIM and removal deltas 318 instead of 575 us.  Four blocks per SM (64 registers): with
-// three or five the latter takes 322 us.
+// warp, which sums its sites' gradients by itself (warp_sums.cuh); with few sites 16x16 pixels
+// per block and a key table (kTable).  Bound by issue (SM 64%, L1 63%): 149 us at 1237x941 with
+// 18,187 sites, SSIM and removal deltas.  A torch step (render, gradients, tau diffusion, Adam,
+// candidate refresh) at 768x512 with 24,576 sites takes 205-215 us, 297 us with a key table and
+// float adds in shared memory; at 1237x941 with SSIM and removal deltas 319 instead of 575 us.
+// Four blocks per SM (64 registers): with three or five the latter took 322 us, with four 318.
 template <class Src, bool kRemoval, bool kSSIM, bool kTable>
 __global__ void __launch_bounds__(256, 4)
     fused_gradients_kernel(const __grid_constant__ GradParams prm, Src src) {

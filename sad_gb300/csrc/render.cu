@@ -196,11 +196,12 @@ void launch_clear_candidates(uint32_t* c0, uint32_t* c1, int w, int h, cudaStrea
 // ---------------------------------------------------------------------------
 // autograd adjoint (backends/pytorch/torch_ext/cuda/sad_bindings.cu:41-207)
 // ---------------------------------------------------------------------------
-// Each warp takes an 8x4 patch and sums its sites' gradients by itself (warp_sums.cuh).  Bound
-// by issue (SM 68%, L1 66%): 290 us at 1999x1503 from the records of 46,941 sites, and at 512x512
-// with 16,384 raw ones 50 us with the operator around it, against 875 and 99 us with a key table
-// and float adds in shared memory.  Four blocks per SM (64 registers): a render and its adjoint
-// at 1999x1503 take 372 us, with three 415 us, with five 382 us.
+// Each warp takes an 8x4 patch and sums its sites' gradients by itself (warp_sums.cuh); with few
+// sites through a key table (kTable).  Bound by issue (SM 68%, L1 68%): 296 us at 1999x1503 from
+// the records of 46,941 sites, and at 512x512 with 16,384 raw ones 50 us with the operator around
+// it, against 875 and 99 us with a key table and float adds in shared memory.  Four blocks per SM
+// (64 registers): a render and its adjoint at 1999x1503 took 372 us (378 now), with three 415 us,
+// with five 382 us.
 template <class Src, bool kTable>
 __global__ void __launch_bounds__(256, 4) render_backward_kernel(
     const uint4* __restrict__ cand0, const uint4* __restrict__ cand1,

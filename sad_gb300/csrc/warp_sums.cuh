@@ -6,14 +6,14 @@
 // whose 64 candidates name some 10-20 distinct sites) takes one site after the other, the
 // smallest id left first: the lanes that list it compute their terms, a folding butterfly
 // sums them over the group and leaves each lane two of the sums at most, which go to global
-// memory by one reduction per value.  No add in shared memory, and one barrier in the block.
+// memory by one reduction per value.  No add in shared memory.
 // What is the same for every pixel of a site (softness, scales) is multiplied in after the
 // sum.  Groups of 8 balance the site loop's length, which falls with the group (fewer
 // distinct sites, fewer idle lanes), against the global reductions, which rise: a 1999x1503
-// render and its adjoint take 372 us, with groups of 4 and 16 lanes 481 and 468 us.
+// render and its adjoint took 372 us (378 now), with groups of 4 and 16 lanes 481 and 468 us.
 // A lane sorts its list by id first (19 exchanges), so that the loop compares and shifts its
 // head instead of scanning eight ids for the minimum and for each match (some 20 of 150
-// instructions a round): 372 instead of 394 us there from site records; step at 1237x941 with
+// instructions a round): 372 instead of 394 us there from site records; a step at 1237x941 with
 // SSIM and removal deltas 325 instead of 328 us.
 // Lists with little in common (a random initial field) would make that loop long: a block with
 // such a group (kMostMarks) takes a key table in shared memory instead, whose float adds rarely
@@ -32,7 +32,7 @@ constexpr int kSumSlots = 512;  // keys of the block's table
 
 // Whether all sums go through the table: with few sites on many pixels the groups' reductions
 // queue up at the same addresses in L2 (1999x1503 with 64 sites: the adjoint 2775 us, 759 by
-// table; the gradients with SSIM and removal deltas 3978 and 899 us), and a table holds every
+// table; the gradients with SSIM and removal deltas 3978 and 893 us), and a table holds every
 // site.  The line lies where the two meet on nearest-site fields: at one site per `per_site`
 // pixels on small images and at `most` sites on large ones.  Adjoint by groups and by table: at
 // 256x256 with 64 sites 75 and 45 us, with 100 sites 48 and 46; at 1024x1024 with 300 sites 362 and
@@ -162,9 +162,8 @@ __device__ __forceinline__ void sort_candidates(uint32_t (&ids)[kCand], float (&
 // How many of 64 hash values the ids of the lane's group take: 64 (1 - e^(-d/64)) for d distinct
 // ids, give or take two.  Some 27 sites, or rounds of the loop, are its limit, which a field of
 // one site a pixel still keeps: the adjoint at 256x256 with 65,536 sites takes 25 us with a
-// limit of 22 marks, 46 with 19; at 512x512 with 262,144 sites 52 and 72 us; from random lists
-// of 256 sites at 181x181, where the longest loop counts, 41 us, with a limit of 25 marks the
-// same, of 19 marks 39 us.
+// limit of 22 marks, 46 with 19; at 512x512 with 262,144 sites 52 and 72 us; with a limit of
+// 25 both the same.
 constexpr int kMostMarks = 22;
 __device__ __forceinline__ int distinct_marks(const uint32_t (&ids)[kCand]) {
     uint32_t lo = 0u, hi = 0u;

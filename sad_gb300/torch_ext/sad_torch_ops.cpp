@@ -60,7 +60,11 @@ T* ptr(const Tensor& t) {
 uint32_t u32(int64_t v) { return static_cast<uint32_t>(v); }
 
 // Whether site records, built once per call by a launch of their own, pay for themselves in a
-// kernel over `pixels` that reads eight sites each.
+// kernel over `pixels` that reads eight sites each.  Kernels without and with records, one site
+// per 16 pixels: at 131,072 pixels the render 9 and 10 us, the adjoint 27 and 25, gradients 39 and
+// 38; at 262,144 pixels 14 and 11, 44 and 42, 60 and 58; at 524,288 pixels 23 and 19, 78 and 70,
+// 102 and 98; at 1,048,576 pixels 35 and 28, 122 and 107, 160 and 153.  The line lies above the
+// sizes whose calls are bound by the host, which pays for the scratch and the second launch.
 constexpr int64_t kRecordPixels = 1 << 19;
 bool records_pay(int64_t pixels, int64_t sites) { return pixels >= kRecordPixels && sites <= pixels; }
 
@@ -230,6 +234,10 @@ Tensor pack_candidate_sites(const Tensor& sites_, const Tensor& packed_, int64_t
     return packed;
 }
 
+// The same for a candidate pass, against decoding packed sites at every visit: the line lies where
+// the two meet (one site per 16 texels: 65,536 texels 15.0 and 16.8 us, 131,072 texels 16.7 and
+// 17.0, 262,144 texels 27.4 and 26.9, 524,288 texels 49.8 and 44.8; on fewer sites it is later:
+// 131,072 texels with 2,048 sites 14.8 and 16.5).
 constexpr int64_t kRecordTexels = 1 << 17;
 
 // sad_bindings.cu:786-863
